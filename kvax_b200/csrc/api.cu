@@ -92,7 +92,7 @@ int mask_view(const kvax_b200_block_mask& m, bool kv_outer, int q_len, int kv_le
   return KVAX_B200_OK;
 }
 
-struct ListLayout { size_t tiles_off, counts_off, order_off, bitmaps_off, total; int n_outer, n_inner, batch; bool bitmaps; };
+struct ListLayout { size_t tiles_off, counts_off, order_off, bitmaps_off, total; int n_outer, n_inner, batch, tile_bits, n_bitmaps; };
 
 ListLayout list_layout(int batch, int outer_len, int inner_len, size_t base, bool bitmaps = false) {
   ListLayout l;
@@ -103,37 +103,44 @@ ListLayout list_layout(int batch, int outer_len, int inner_len, size_t base, boo
   l.order_off = l.counts_off + align256(size_t(batch) * l.n_outer * sizeof(int32_t));
   // launch order of the single tiles, then of the pairs of neighbouring tiles (the forward's work items)
   l.bitmaps_off = l.order_off + align256(size_t(batch) * (l.n_outer + (l.n_outer + 1) / 2) * sizeof(int32_t));
-  l.bitmaps = bitmaps;
-  // element masks of the first partial entries of every list (attn_common.cuh)
-  l.total = l.bitmaps_off + (bitmaps ? align256(size_t(batch) * l.n_outer * kBitmapSlots * kTile * sizeof(uint4)) : 0);
+  // pool of element masks (attn_common.cuh); an entry's tile and mask index share 30 bits, all ones is left out
+  l.tile_bits = 1;
+  while ((1ll << l.tile_bits) < l.n_inner) ++l.tile_bits;
+  const long long want = (long long)batch * l.n_outer * kBitmapsPerList, most = (1ll << (30 - l.tile_bits)) - 1;
+  l.n_bitmaps = bitmaps ? int(want < most ? want : most) : 0;
+  l.total = l.bitmaps_off + align256(size_t(l.n_bitmaps) * kTile * sizeof(uint4));
   return l;
 }
 
-// per-tile summaries of both sides: query tiles first, kv tiles after
-struct SummaryLayout { size_t q_off, kv_off, total; };
+// per-tile summaries of both sides: query tiles first, kv tiles after, then the list builder's counters
+struct SummaryLayout { size_t q_off, kv_off, counters_off, total; };
 SummaryLayout summary_layout(int batch, int q_len, int kv_len, size_t base) {
   SummaryLayout l;
   l.q_off = base;
   l.kv_off = l.q_off + align256(size_t(batch) * cdiv(q_len, kTile) * sizeof(int4));
-  l.total = l.kv_off + align256(size_t(batch) * cdiv(kv_len, kTile) * sizeof(int4));
+  l.counters_off = l.kv_off + align256(size_t(batch) * cdiv(kv_len, kTile) * sizeof(int4));
+  l.total = l.counters_off + align256(kListCounters * sizeof(int32_t));
   return l;
 }
 
 void fill_schedule(ScheduleArgs* sa, const MaskView& mv, const TokenInfo& tok, char* ws, const ListLayout& ll,
-                   const int4* inner_summary, int outer_len, int inner_len) {
+                   const int4* inner_summary, int32_t* counters, int outer_len, int inner_len) {
   sa->mask = mv; sa->tok = tok;
   sa->tiles = reinterpret_cast<uint32_t*>(ws + ll.tiles_off);
   sa->counts = reinterpret_cast<int32_t*>(ws + ll.counts_off);
   sa->order = reinterpret_cast<int32_t*>(ws + ll.order_off);
   sa->pair_order = sa->order + size_t(ll.batch) * ll.n_outer;
   sa->inner_summary = inner_summary;
-  sa->bitmaps = ll.bitmaps ? reinterpret_cast<uint4*>(ws + ll.bitmaps_off) : nullptr;
+  sa->counters = counters;
+  sa->bitmaps = ll.n_bitmaps ? reinterpret_cast<uint4*>(ws + ll.bitmaps_off) : nullptr;
+  sa->n_bitmaps = ll.n_bitmaps; sa->tile_bits = ll.tile_bits;
   sa->n_outer_tiles = ll.n_outer; sa->n_inner_tiles = ll.n_inner;
   sa->outer_len = outer_len; sa->inner_len = inner_len;
 }
 
 void fill_list(TileList* l, const ScheduleArgs& sa) {
   l->tiles = sa.tiles; l->counts = sa.counts; l->order = sa.order; l->pair_order = sa.pair_order; l->bitmaps = sa.bitmaps;
+  l->tile_bits = sa.tile_bits; l->tile_mask = (1u << sa.tile_bits) - 1;
   l->n_outer_tiles = sa.n_outer_tiles; l->n_inner_tiles = sa.n_inner_tiles;
 }
 
@@ -185,10 +192,11 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   ScheduleArgs sa;
   int4* q_sum = reinterpret_cast<int4*>(ws + sl.q_off);
   int4* kv_sum = reinterpret_cast<int4*>(ws + sl.kv_off);
-  fill_schedule(&sa, mv, token_info(s), ws, ll, kv_sum, s.q_len, s.kv_len);
+  int32_t* counters = reinterpret_cast<int32_t*>(ws + sl.counters_off);
+  fill_schedule(&sa, mv, token_info(s), ws, ll, kv_sum, counters, s.q_len, s.kv_len);
   const int stages = p->stages ? p->stages : 3;
   if (stages & 1) {
-    launch_tile_summaries(sa.tok, s.batch, q_sum, kv_sum, st);
+    launch_tile_summaries(sa.tok, s.batch, q_sum, kv_sum, counters, st);
     launch_schedule(false, sa, s.batch, st);
     if (cudaGetLastError() != cudaSuccess) return KVAX_B200_ELAUNCH;
   }
@@ -297,12 +305,13 @@ extern "C" int kvax_b200_attn_bwd(const kvax_b200_attn_bwd_params* p, void* work
   int4* q_sum = reinterpret_cast<int4*>(ws + bl.sum.q_off);
   int4* kv_sum = reinterpret_cast<int4*>(ws + bl.sum.kv_off);
   ScheduleArgs sq, sk;
-  fill_schedule(&sq, mv_dq, tok, ws, bl.dq, kv_sum, s.q_len, s.kv_len);
-  fill_schedule(&sk, mv_dkdv, tok, ws, bl.dkdv, q_sum, s.kv_len, s.q_len);
+  int32_t* counters = reinterpret_cast<int32_t*>(ws + bl.sum.counters_off);
+  fill_schedule(&sq, mv_dq, tok, ws, bl.dq, kv_sum, counters, s.q_len, s.kv_len);
+  fill_schedule(&sk, mv_dkdv, tok, ws, bl.dkdv, q_sum, counters + 2, s.kv_len, s.q_len);
   const int all = bl.fused ? (1 | 2 | 16 | 32) : (1 | 2 | 4 | 8);
   const int stages = p->stages ? (p->stages & all) : all;
   if (stages & 1) {
-    launch_tile_summaries(tok, s.batch, q_sum, kv_sum, st);
+    launch_tile_summaries(tok, s.batch, q_sum, kv_sum, counters, st);
     if (!bl.fused) launch_schedule(false, sq, s.batch, st);       // the fused kernel only walks the kv-outer lists
     launch_schedule(true, sk, s.batch, st);
   }

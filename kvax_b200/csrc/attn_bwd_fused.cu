@@ -99,7 +99,7 @@ struct FusedSmem {
 };
 
 // Mask bits of kv row r for the 64 queries [i0, i0 + 64) of a partial list entry that carries no element mask from the
-// list builder (more than kBitmapSlots partial entries in one list: rare).  Deliberately not inlined: what it needs --
+// list builder (its pool of masks was used up: rare).  Deliberately not inlined: what it needs --
 // the row's bounds, its segment id and position, the query arrays -- then lives in no register of the item loop (a
 // build of the loop that took every mask from the list builder ran 4 % faster than one that could also compute them).
 __device__ __noinline__ uint2 fused_keep_slow(const BwdArgs* a, int b, int r, int i0) {
@@ -210,7 +210,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     PH_BEGIN()
     for (int i = 0; i < n && ok; ++i) {
       const int st = i & 1;
-      const int u = int(e_next & kTileIndexMask);
+      const int u = int(e_next & a.list.tile_mask);
       const int yh = qh;
       if (++li == cnt) { li = 0; ++qh; }
       if (i + 1 < n) e_next = __ldg(list + li);
@@ -380,12 +380,11 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     const uint32_t my_t1 = tT1 + lane_base + cb;              // fp32 columns of this thread; P^T goes to the first 32 of them
     const uint32_t my_t2 = tT2 + lane_base + cb;
     const float c = a.scale_log2e;
-    // Mask bits of this thread's 64 queries of partial list entry e: the element mask the list builder worked out for
-    // the first partial entries of every list (one 8-byte load), else computed by the function above.
-    const uint2* bitmap_row = reinterpret_cast<const uint2*>(a.list.bitmaps + (list_row * kBitmapSlots) * kTile + row) + half;
+    // Mask bits of this thread's 64 queries of partial list entry e: the element mask the list builder worked out (one
+    // 8-byte load), else computed by the function above.
     auto item_keep = [&](uint32_t e, uint32_t* k2) {
-      const uint2 w = (e & kBitmapBit) ? __ldg(bitmap_row + ((e >> kBitmapSlotShift) & (kBitmapSlots - 1)) * (kTile * 2))
-                                       : fused_keep_slow(&a, b, r, int(e & kTileIndexMask) * kTile + cb);
+      const uint2 w = (e & kBitmapBit) ? __ldg(reinterpret_cast<const uint2*>(entry_bitmap(a.list, e) + row) + half)
+                                       : fused_keep_slow(&a, b, r, int(e & a.list.tile_mask) * kTile + cb);
       k2[0] = w.x; k2[1] = w.y;
     };
 
@@ -553,7 +552,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     int li = 0, qh = first_head;
     PH_BEGIN()
     for (int i = 0; i < n_items && ok; ++i) {
-      const int q0 = int(e_next & kTileIndexMask) * kTile + dw * 32;    // first query row this warp drains
+      const int q0 = int(e_next & a.list.tile_mask) * kTile + dw * 32;    // first query row this warp drains
       const int yh = qh;
       if (++li == count) { li = 0; ++qh; }
       if (i + 1 < n_items) e_next = ldg_pinned(list + li);

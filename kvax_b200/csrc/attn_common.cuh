@@ -11,14 +11,14 @@ namespace kvx {
 constexpr int kTile = 128;                 // native tile edge of every attention kernel
 constexpr uint32_t kPartialBit = 0x80000000u;
 // Element masks of partial tiles depend on (batch row, outer tile, inner tile) only, not on the head: the list builder
-// works out the first kBitmapSlots of every list once -- 128 rows x 128 bits, one uint4 per outer row -- and marks
-// those entries; the attention kernels then load 16 bytes per row and tile instead of comparing 128 segment ids and
-// positions per row, tile and head.  Further partial entries of a list are masked by the consumer as before.
-// A marked entry carries its slot: bit 31 partial, bit 30 marked, bits 27-29 the slot, bits 0-26 the inner tile.
+// works each out once -- 128 rows x 128 bits, one uint4 per outer row -- and the attention kernels load 16 bytes per row and
+// tile instead of comparing 128 segment ids and positions per row, tile and head.  The masks of all lists share one pool
+// of kBitmapsPerList masks per list on average (a list of a packed batch has two or three partial entries, but a query
+// tile that holds the end of a long document has one per kv tile of it); once the pool is used up, further partial
+// entries are masked by the consumer.  A list entry: bit 31 partial, bit 30 has a mask, the low `tile_bits` bits the inner
+// tile, the bits in between the mask's index in the pool.
 constexpr uint32_t kBitmapBit = 0x40000000u;
-constexpr int kBitmapSlotShift = 27;
-constexpr uint32_t kTileIndexMask = 0x07ffffffu;
-constexpr int kBitmapSlots = 8;
+constexpr int kBitmapsPerList = 8;
 
 // Block mask plus the geometry needed to read it.
 struct MaskView {
@@ -180,9 +180,16 @@ struct TileList {
   const int32_t* counts;   // (B, n_outer_tiles)
   const int32_t* order;    // (B * n_outer_tiles) launch order: row = b * n_outer_tiles + tile
   const int32_t* pair_order;   // (B * ceil(n_outer_tiles / 2)) launch order of the pairs (2p, 2p+1): row of tile 2p
-  const uint4* bitmaps;        // (B * n_outer_tiles, kBitmapSlots, 128) element masks of marked entries, or null: none marked
+  const uint4* bitmaps;        // (pool, 128) element masks of marked entries, or null: none marked
+  uint32_t tile_mask;          // low `tile_bits` bits of an entry
+  int32_t tile_bits;
   int32_t n_outer_tiles, n_inner_tiles;
 };
+
+// The element mask of a marked entry.
+__device__ __forceinline__ const uint4* entry_bitmap(const TileList& l, uint32_t e) {
+  return l.bitmaps + (long long)((e & (kBitmapBit - 1)) >> l.tile_bits) * kTile;
+}
 
 // Launch geometry shared by the attention kernels: a 1-D grid over (outer tile, head).
 // Outer tiles are taken in the launch order built by schedule.cu (blocks of kRowChunk

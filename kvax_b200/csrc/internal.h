@@ -9,6 +9,8 @@
 
 namespace kvx {
 
+constexpr int kListCounters = 4;   // two per list of a call (the backward builds up to two)
+
 struct ScheduleArgs {
   MaskView mask;
   TokenInfo tok;
@@ -17,11 +19,13 @@ struct ScheduleArgs {
   int32_t* order;      // (B * n_outer_tiles) launch order of the rows (blocks of neighbours, longest lists first)
   int32_t* pair_order; // (B * ceil(n_outer_tiles / 2)) the same order for pairs (2p, 2p+1): row of the even tile
   const int4* inner_summary;  // (B, n_inner_tiles) {seg_min, seg_max, pos_min, pos_max}
-  uint4* bitmaps;      // (B * n_outer_tiles, kBitmapSlots, 128) element masks of the first partial entries of a list, or null
+  int32_t* counters;   // [0] masks taken from the pool, [1] finished lists; zero on entry (launch_tile_summaries)
+  uint4* bitmaps;      // (n_bitmaps, 128) pool of element masks, or null
+  int32_t n_bitmaps, tile_bits;
   int32_t n_outer_tiles, n_inner_tiles;
   int32_t outer_len, inner_len;
 };
-void launch_tile_summaries(const TokenInfo& tok, int batch, int4* q_sum, int4* kv_sum, cudaStream_t s);
+void launch_tile_summaries(const TokenInfo& tok, int batch, int4* q_sum, int4* kv_sum, int32_t* counters, cudaStream_t s);
 void launch_schedule(bool kv_outer, const ScheduleArgs& a, int batch, cudaStream_t s);
 
 struct FwdArgs {

@@ -2,17 +2,30 @@
 // into, for every 128-row outer tile, the ascending list of 128-column inner tiles the
 // attention kernels must visit, plus a longest-first launch order of the outer tiles.
 //
-//   * A tile whose every element lies in the "full" range of every row is emitted as
-//     unmasked.
+//   * A tile whose every element is allowed is emitted as unmasked.
 //   * A tile in which no element survives the reference's element-level rule is dropped
-//     (it contributes nothing to any row).  Most such tiles are rejected by an interval
-//     test on per-tile (segment min/max, position min/max) summaries; the rest by an exact
-//     128 x 128 test.
-//   * Everything else is emitted as partial and masked per element by the consumer.
+//     (it contributes nothing to any row).
+//   * Everything else is emitted as partial, with its element mask (128 x 128 bits) in a
+//     pool of kBitmapsPerList masks per list on average; once the pool is full, further
+//     partial tiles are masked per element by the consumer.
 //
-// Launches: tile_summary_kernel (one warp per 128-token tile of either side),
-// schedule_kernel (one CTA of 128 threads per (outer tile, batch); thread t owns outer
-// row t), order_kernel (one CTA: counting sort of the outer tiles by list length).
+// Launches: tile_summary_kernel (one warp per 128-token tile of either side) and
+// schedule_kernel (one CTA of sixteen warps per (outer tile, batch)).  What bounds the builder
+// is latency, not bytes or arithmetic, so the work of a list is spread over lanes and warps:
+//   A  one lane per inner tile: interval test of the tile's summary against the outer tile's
+//      ranges of bounds, segments and positions.  Decides most tiles.
+//   B  one warp per undecided tile: the exact element mask.  A lane owns four outer rows.  The
+//      128 inner tokens are cut into runs of one segment with consecutive positions (packed
+//      documents: one to three runs per tile); inside a run the allowed tokens of a row are an
+//      interval, so a row costs a few integer operations per run instead of 128 comparisons.
+//      Tiles with more than kMaxRuns runs compare token by token.
+//   C  ordered compaction.
+// The CTA that finishes last sorts the outer tiles into the launch order, which saves a launch.
+// Measured against one CTA of 128 threads per list that compared element by element and an order kernel of its own:
+// 69 -> 13 us (1 x 8k tokens, packed), 97 -> 30 us (2 x 32k, packed), 134 -> 13 us (2 x 5003, packed, rows off the 16-byte
+// grid), 53 -> 15 us (one query tile against 64 kv tiles, batch 16).  Before, only the first eight partial tiles of a list
+// had their masks worked out here, and a query tile cut by the end of the sequence was partial throughout: the forward kernel
+// compared token ids itself on those, 560 -> 320 us for 2 x 5003 tokens and 656 -> 231 us for one query against 8k keys.
 #include "attn_common.cuh"
 #include "internal.h"
 
@@ -20,13 +33,16 @@ namespace kvx {
 
 namespace {
 
-constexpr int kChunk = 1024;   // inner tiles classified per pass
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kChunk = kThreads;   // inner tiles classified per pass: one per thread
+constexpr int kMaxRuns = 16;       // a run costs a row about 40 operations, comparing token by token about 600
 
 // ---- per-tile summaries ---------------------------------------------------------------
 // int4 {seg_min, seg_max, pos_min, pos_max} over the valid tokens of a tile; raw segment
 // ids (PAD participates: PAD matches PAD in the element rule).
 __global__ void __launch_bounds__(256) tile_summary_kernel(const TokenInfo tok, int4* q_sum, int4* kv_sum,
-                                                          int n_q_tiles, int n_kv_tiles, int batch) {
+                                                          int n_q_tiles, int n_kv_tiles, int batch, int32_t* counters) {
+  if (blockIdx.x == 0 && threadIdx.x < kListCounters) counters[threadIdx.x] = 0;
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_q = (long long)batch * n_q_tiles, n_all = n_q + (long long)batch * n_kv_tiles;
@@ -48,186 +64,6 @@ __global__ void __launch_bounds__(256) tile_summary_kernel(const TokenInfo tok, 
   if (lane == 0) (is_q ? q_sum : kv_sum)[local] = make_int4(smin, smax, pmin, pmax);
 }
 
-__device__ __forceinline__ int block_min(int v, int* s) {
-  v = __reduce_min_sync(0xffffffffu, v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  return min(min(s[0], s[1]), min(s[2], s[3]));
-}
-__device__ __forceinline__ int block_max(int v, int* s) {
-  v = __reduce_max_sync(0xffffffffu, v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  return max(max(s[0], s[1]), max(s[2], s[3]));
-}
-
-template <bool kKvOuter>
-__global__ void __launch_bounds__(kTile) schedule_kernel(const ScheduleArgs a) {
-  __shared__ int s_seg[kTile];
-  __shared__ int s_pos[kTile];
-  __shared__ int s_red[4];
-  __shared__ int s_red2[4];
-  __shared__ unsigned char s_code[kChunk];    // 0 drop, 1 unmasked, 2 needs the exact test, 3 partial
-  __shared__ int s_count;
-  __shared__ int s_partial;                   // partial entries of the list so far
-  __shared__ int s_slot_tile[kBitmapSlots];   // inner tile of the partial entry that got bitmap slot i
-  const int t = threadIdx.x;
-  const int ot = blockIdx.x, b = blockIdx.y;
-  const int o = ot * kTile + t;                       // outer token of this thread
-  const bool row_valid = o < a.outer_len;
-
-  const RowBounds rb = load_bounds(a.mask, b, min(o, a.outer_len - 1));
-  int o_seg = KVAX_B200_PADDING_SEGMENT_ID, o_pos = 0;
-  if (row_valid) {
-    if (kKvOuter) {
-      o_seg = __ldg(a.tok.kv_seg + (long long)b * a.tok.kv_len + o);
-      o_pos = a.tok.sequential ? o : __ldg(a.tok.kv_pos + (long long)b * a.tok.kv_len + o);
-    } else {
-      o_seg = __ldg(a.tok.q_seg + (long long)b * a.tok.q_len + o);
-      o_pos = query_position(a.tok, b, o);
-    }
-  }
-
-  // CTA-wide ranges on the inner axis (tokens)
-  const bool visits = row_valid && rb.up > rb.lo;
-  const bool has_full = row_valid && rb.uf > rb.lof;
-  const int vis_lo = block_min(visits ? rb.lo : INT32_MAX, s_red);
-  int vis_hi = block_max(visits ? rb.up : 0, s_red);
-  const int all_full_lo = block_max(row_valid ? rb.lof : 0, s_red);         // full for every row
-  const int all_full_hi = min(block_min(row_valid ? rb.uf : INT32_MAX, s_red), a.inner_len);
-  vis_hi = min(vis_hi, a.n_inner_tiles * kTile);
-
-  uint32_t* out = a.tiles + ((long long)b * a.n_outer_tiles + ot) * a.n_inner_tiles;
-  if (t == 0) { s_count = 0; s_partial = 0; }
-  __syncthreads();
-  if (vis_hi > vis_lo) {
-    const int it0 = max(vis_lo, 0) / kTile;
-    const int it1 = min((vis_hi + kTile - 1) / kTile, a.n_inner_tiles);
-    const int4* inner_sum = a.inner_summary + (long long)b * a.n_inner_tiles;
-    for (int base = it0; base < it1; base += kChunk) {
-      const int n = min(kChunk, it1 - base);
-      // A: interval classification.  Every thread tests its own row against the summary
-      // of 32 inner tiles at a time; a tile stays a candidate when any row may hold an
-      // allowed element in it.
-      for (int k0 = 0; k0 < n; k0 += 32) {
-        uint32_t pass = 0, sure = 0;
-        if (row_valid) {
-          const int kn = min(32, n - k0);
-          for (int k = 0; k < kn; ++k) {
-            const int c0 = (base + k0 + k) * kTile, c1 = c0 + kTile;
-            const int4 s = __ldg(inner_sum + base + k0 + k);      // {smin, smax, pmin, pmax}
-            const bool in_full = (c0 < rb.uf) && (c1 > rb.lof);
-            const bool seg_in = (s.x <= o_seg) && (o_seg <= s.y);
-            const bool left_ov = (c0 < rb.lof) && (c1 > rb.lo);
-            const bool right_ov = (c0 < rb.up) && (c1 > rb.uf);
-            const bool causal_ok = kKvOuter ? (s.w >= o_pos) : (o_pos >= s.z);
-            const bool cls = kKvOuter ? (right_ov || (left_ov && causal_ok)) : (left_ov || (right_ov && causal_ok));
-            pass |= ((in_full || (seg_in && cls)) ? 1u : 0u) << k;
-            // sufficient condition for "this row has an allowed element in the tile": part of
-            // the tile lies in the row's full range, or the tile is one segment equal to the
-            // row's, lies inside one class of the row and (where that class is causal) every
-            // position in it passes the causal test
-            const bool full_hit = in_full && (max(c0, rb.lof) < a.inner_len);
-            const bool single = (s.x == s.y) && (s.x == o_seg);
-            const bool left_all = (c0 >= rb.lo) && (c1 <= rb.lof);
-            const bool right_all = (c0 >= rb.uf) && (c1 <= rb.up);
-            const bool causal_all = kKvOuter ? (s.z >= o_pos) : (o_pos >= s.w);
-            const bool cls_all = kKvOuter ? (right_all || (left_all && causal_all)) : (left_all || (right_all && causal_all));
-            sure |= ((full_hit || (single && cls_all)) ? 1u : 0u) << k;
-          }
-        }
-        pass = __reduce_or_sync(0xffffffffu, pass);
-        sure = __reduce_or_sync(0xffffffffu, sure);
-        __syncthreads();
-        if ((t & 31) == 0) { s_red[t >> 5] = int(pass); s_red2[t >> 5] = int(sure); }
-        __syncthreads();
-        if (t < 32 && k0 + t < n) {
-          const uint32_t any = uint32_t(s_red[0] | s_red[1] | s_red[2] | s_red[3]);
-          const uint32_t any_sure = uint32_t(s_red2[0] | s_red2[1] | s_red2[2] | s_red2[3]);
-          const int c0 = (base + k0 + t) * kTile;
-          s_code[k0 + t] = (all_full_lo <= c0 && c0 + kTile <= all_full_hi) ? 1
-                           : (((any_sure >> t) & 1u) ? 3 : (((any >> t) & 1u) ? 2 : 0));
-        }
-      }
-      __syncthreads();
-      // B: exact test of the undecided tiles (CTA-wide, thread t scans the columns for row t)
-      for (int k = 0; k < n; ++k) {
-        if (s_code[k] != 2) continue;                       // uniform: shared memory value
-        const int c0 = (base + k) * kTile;
-        const int i = c0 + t;
-        int seg = KVAX_B200_PADDING_SEGMENT_ID, pos = 0;
-        if (i < a.inner_len) {
-          if (kKvOuter) {
-            seg = __ldg(a.tok.q_seg + (long long)b * a.tok.q_len + i);
-            pos = query_position(a.tok, b, i);
-          } else {
-            seg = __ldg(a.tok.kv_seg + (long long)b * a.tok.kv_len + i);
-            pos = a.tok.sequential ? i : __ldg(a.tok.kv_pos + (long long)b * a.tok.kv_len + i);
-          }
-        }
-        s_seg[t] = seg; s_pos[t] = pos;
-        __syncthreads();
-        int found = 0;
-        if (row_valid) {
-          const int lim = min(kTile, a.inner_len - c0);
-          for (int j = 0; j < lim; ++j) {
-            const bool seg_eq = (s_seg[j] == o_seg);
-            const bool causal = kKvOuter ? (s_pos[j] >= o_pos) : (o_pos >= s_pos[j]);
-            if (element_allowed<kKvOuter>(rb, c0 + j, seg_eq, causal)) { found = 1; break; }
-          }
-        }
-        const int any = __syncthreads_or(found);
-        if (t == 0) s_code[k] = any ? 3 : 0;
-      }
-      __syncthreads();
-      // C: ordered compaction by warp 0.  The first kBitmapSlots partial entries of a list get an element
-      // mask of their own (step D) and are marked.
-      const bool with_bitmaps = a.bitmaps != nullptr;
-      const int partial_before = s_partial;
-      if (t < 32) {
-        int cnt = s_count, pcnt = partial_before;
-        for (int k0 = 0; k0 < n; k0 += 32) {
-          const int k = k0 + t;
-          const unsigned char code = (k < n) ? s_code[k] : 0;
-          const unsigned m = __ballot_sync(0xffffffffu, code != 0);
-          const unsigned pm = __ballot_sync(0xffffffffu, code == 3);
-          if (code != 0) {
-            uint32_t e = uint32_t(base + k) | (code == 3 ? kPartialBit : 0u);
-            const int slot = pcnt + __popc(pm & ((1u << t) - 1));
-            if (code == 3 && with_bitmaps && slot < kBitmapSlots) { e |= kBitmapBit | (uint32_t(slot) << kBitmapSlotShift); s_slot_tile[slot] = base + k; }
-            out[cnt + __popc(m & ((1u << t) - 1))] = e;
-          }
-          cnt += __popc(m);
-          pcnt += __popc(pm);
-        }
-        if (t == 0) { s_count = cnt; s_partial = pcnt; }
-      }
-      __syncthreads();
-      // D: element masks of the entries marked in this pass: thread t = outer row t, the very function the consumers
-      // would call on the same arguments
-      if (with_bitmaps) {
-        const int slot_end = min(s_partial, kBitmapSlots);
-        const int32_t* inner_seg = a.tok.kv_seg + (long long)b * a.tok.kv_len;
-        const int32_t* inner_pos = a.tok.sequential ? nullptr : a.tok.kv_pos + (long long)b * a.tok.kv_len;
-        for (int slot = partial_before; slot < slot_end; ++slot) {
-          const int c0 = s_slot_tile[slot] * kTile;
-          uint32_t w[4];
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch)
-            w[ch] = kKvOuter ? kv_outer_keep32(a.tok, rb, b, row_valid, o_seg, o_pos, c0 + ch * 32)
-                             : keep_bits32<false>(rb, c0 + ch * 32, a.inner_len, row_valid, o_seg, o_pos, inner_seg + c0 + ch * 32,
-                                                  inner_pos ? inner_pos + c0 + ch * 32 : nullptr);
-          a.bitmaps[(((long long)b * a.n_outer_tiles + ot) * kBitmapSlots + slot) * kTile + t] = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-        __syncthreads();                        // s_slot_tile is reused by the next pass
-      }
-    }
-  }
-  if (t == 0) a.counts[(long long)b * a.n_outer_tiles + ot] = s_count;
-}
-
 // Launch order.  Outer tiles are launched in blocks of kRowChunk neighbours (same batch row, consecutive tile
 // indices), the blocks sorted by their mean list length, longest first: the tail of a launch is then made of short
 // work items, and the CTAs that are resident together belong to neighbouring outer tiles of a few heads, which walk
@@ -235,85 +71,335 @@ __global__ void __launch_bounds__(kTile) schedule_kernel(const ScheduleArgs a) {
 // fall on dQ accumulator lines that are still there.  (Sorting single tiles by length instead mixes the documents
 // of a batch: measured 22 GB of DRAM traffic per fused-backward launch on the 32k workload for 3 GB of algorithmic bytes.)
 // Counting sort of the blocks in one CTA; the order among blocks of equal key is not fixed.
-constexpr int kBins = 2048;                // two per thread of order_kernel
-__global__ void __launch_bounds__(1024) order_kernel(const int32_t* counts, int32_t* order, int32_t* pair_order, int n_outer,
-                                                     int batch) {
-  __shared__ int hist[kBins];        // rows per key, then the running start of the key's rows
-  __shared__ int hist2[kBins];       // the same in units of pairs of neighbouring rows
+constexpr int kBins = 2048;                // four per thread
+static_assert(kBins == 4 * kThreads, "the scan below takes four bins per thread");
+struct OrderSmem {
+  int hist[kBins];         // rows per key, then the running start of the key's rows
+  int hist2[kBins];        // the same in units of pairs of neighbouring rows
+  int warp_tot[kWarps], warp_tot2[kWarps];
+};
+
+__device__ void launch_order(OrderSmem& sm, const int32_t* counts, int32_t* order, int32_t* pair_order, int n_outer, int batch) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int blocks_per_row = (n_outer + kRowChunk - 1) / kRowChunk;
   const int n_blocks = blocks_per_row * batch;
-  auto block_info = [&](int blk, int* first_row, int* rows) -> int {     // returns the key (mean list length, clamped)
+  static_assert(kRowChunk == 32, "one lane per row of a block");
+  // whole warp; returns the key (mean list length, clamped).  The counts come from other CTAs: read past L1.
+  auto block_info = [&](int blk, int* first_row, int* rows) -> int {
     const int b = blk / blocks_per_row, t0 = (blk - b * blocks_per_row) * kRowChunk;
     const int n = min(kRowChunk, n_outer - t0);
     *first_row = b * n_outer + t0;
     *rows = n;
-    int sum = 0;
-    for (int j = 0; j < n; ++j) sum += counts[*first_row + j];
+    const int sum = __reduce_add_sync(0xffffffffu, lane < n ? __ldcg(counts + *first_row + lane) : 0);
     return min((sum + n - 1) / n, kBins - 1);
   };
-  for (int i = threadIdx.x; i < kBins; i += blockDim.x) { hist[i] = 0; hist2[i] = 0; }
+  for (int i = tid; i < kBins; i += kThreads) { sm.hist[i] = 0; sm.hist2[i] = 0; }
   __syncthreads();
-  for (int blk = threadIdx.x; blk < n_blocks; blk += blockDim.x) {
+  for (int blk = w; blk < n_blocks; blk += kWarps) {
     int first, rows;
     const int key = block_info(blk, &first, &rows);
-    atomicAdd(&hist[key], rows);
-    atomicAdd(&hist2[key], (rows + 1) / 2);
+    if (lane == 0) { atomicAdd(&sm.hist[key], rows); atomicAdd(&sm.hist2[key], (rows + 1) / 2); }
   }
   __syncthreads();
-  // exclusive prefix over descending bins: start[bin] = number of rows in blocks with a larger key.  Thread r takes the
-  // bins kBins - 1 - 2r and kBins - 2 - 2r (two per thread of the 1024), a block-wide scan of the pair sums does the rest.
+  // exclusive prefix over descending bins: start[bin] = number of rows in blocks with a larger key.  Thread r takes four
+  // neighbouring bins from the top down, a block-wide scan of the sums does the rest.
   {
-    __shared__ int warp_tot[32], warp_tot2[32];
-    const int r = threadIdx.x, lane = r & 31, w = r >> 5;
-    const int b0 = kBins - 1 - 2 * r, b1 = b0 - 1;
-    const int c0 = hist[b0], c1 = hist[b1], d0 = hist2[b0], d1 = hist2[b1];
-    int inc = c0 + c1, inc2 = d0 + d1;
+    const int b0 = kBins - 1 - 4 * tid;
+    int c[4], d[4], inc = 0, inc2 = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { c[i] = sm.hist[b0 - i]; d[i] = sm.hist2[b0 - i]; inc += c[i]; inc2 += d[i]; }
+    const int own = inc, own2 = inc2;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, inc, o), t2 = __shfl_up_sync(0xffffffffu, inc2, o);
       if (lane >= o) { inc += t; inc2 += t2; }
     }
-    if (lane == 31) { warp_tot[w] = inc; warp_tot2[w] = inc2; }
+    if (lane == 31) { sm.warp_tot[w] = inc; sm.warp_tot2[w] = inc2; }
     __syncthreads();
-    if (w == 0) {
-      int t = warp_tot[lane], t2 = warp_tot2[lane];
+    int base = inc - own, base2 = inc2 - own2;
+    for (int i = 0; i < w; ++i) { base += sm.warp_tot[i]; base2 += sm.warp_tot2[i]; }
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, t, o), u2 = __shfl_up_sync(0xffffffffu, t2, o);
-        if (lane >= o) { t += u; t2 += u2; }
-      }
-      warp_tot[lane] = t; warp_tot2[lane] = t2;            // inclusive totals of the warps
-    }
-    __syncthreads();
-    const int base = (w ? warp_tot[w - 1] : 0) + inc - (c0 + c1), base2 = (w ? warp_tot2[w - 1] : 0) + inc2 - (d0 + d1);
-    hist[b0] = base; hist[b1] = base + c0;
-    hist2[b0] = base2; hist2[b1] = base2 + d0;
+    for (int i = 0; i < 4; ++i) { sm.hist[b0 - i] = base; sm.hist2[b0 - i] = base2; base += c[i]; base2 += d[i]; }
   }
   __syncthreads();
-  for (int blk = threadIdx.x; blk < n_blocks; blk += blockDim.x) {
+  for (int blk = w; blk < n_blocks; blk += kWarps) {
     int first, rows;
     const int key = block_info(blk, &first, &rows);
-    const int pos = atomicAdd(&hist[key], rows);
-    for (int j = 0; j < rows; ++j) order[pos + j] = first + j;
+    int pos = 0, pos2 = 0;
+    if (lane == 0) { pos = atomicAdd(&sm.hist[key], rows); pos2 = atomicAdd(&sm.hist2[key], (rows + 1) / 2); }
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    pos2 = __shfl_sync(0xffffffffu, pos2, 0);
+    if (lane < rows) order[pos + lane] = first + lane;
     // a block starts at an even tile of its batch row (kRowChunk is even): its pairs are (first + 2j, first + 2j + 1)
-    const int pos2 = atomicAdd(&hist2[key], (rows + 1) / 2);
-    for (int j = 0; j < (rows + 1) / 2; ++j) pair_order[pos2 + j] = first + 2 * j;
+    if (lane < (rows + 1) / 2) pair_order[pos2 + lane] = first + 2 * lane;
+  }
+}
+
+// Bits [a, b) of a 128-bit row mask, in tile coordinates (clamped to the tile).
+__device__ __forceinline__ void add_range(uint32_t (&w)[4], int a, int b) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int s = max(a - 32 * q, 0), n = max(min(b - 32 * q, 32) - s, 0);
+    uint32_t m;
+    asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(m) : "r"(s), "r"(n));
+    w[q] |= m;
+  }
+}
+
+// Mask of one outer row for the 128 inner tokens from c0, token by token.  Not inlined: rare, and large.
+template <bool kKvOuter>
+__device__ __noinline__ uint4 row_mask_by_token(const ScheduleArgs* a, RowBounds rb, int b, bool valid, int seg, int pos, int c0) {
+  const int32_t* kv_seg = a->tok.kv_seg + (long long)b * a->tok.kv_len;
+  const int32_t* kv_pos = a->tok.sequential ? nullptr : a->tok.kv_pos + (long long)b * a->tok.kv_len;
+  uint32_t w[4];
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) {
+    const int i0 = c0 + ch * 32;
+    w[ch] = kKvOuter ? kv_outer_keep32(a->tok, rb, b, valid, seg, pos, i0)
+                     : keep_bits32<false>(rb, i0, a->inner_len, valid, seg, pos, kv_seg + i0, kv_pos ? kv_pos + i0 : nullptr);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+constexpr uint32_t kDropped = 0xffffffffu;   // no list entry: bits 30 and 31 of an entry come with a tile index, and the
+                                             // pool never holds enough masks to set every slot bit as well
+
+template <bool kKvOuter>
+__global__ void __launch_bounds__(kThreads, 2) schedule_kernel(const __grid_constant__ ScheduleArgs a) {
+  __shared__ uint32_t s_entry[kChunk];        // list entry of every inner tile of the pass, or kDropped
+  __shared__ int s_cand[kChunk];              // tiles of the pass that need the exact test
+  __shared__ int s_warp_count[kWarps];
+  __shared__ int s_n_cand, s_last;
+  __shared__ OrderSmem s_order;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ot = blockIdx.x, b = blockIdx.y;
+  const int32_t* inner_seg = (kKvOuter ? a.tok.q_seg : a.tok.kv_seg) + (long long)b * a.inner_len;
+  auto inner_pos = [&](int i) -> int {
+    if (kKvOuter) return query_position(a.tok, b, i);
+    return a.tok.sequential ? i : __ldg(a.tok.kv_pos + (long long)b * a.tok.kv_len + i);
+  };
+
+  // The outer rows ot * 128 + lane + 32 k of this lane (every warp holds all 128 rows), and their joint ranges.
+  RowBounds rb[4];
+  int seg[4], pos[4];
+  bool valid[4];
+  int vis_lo = INT32_MAX, vis_hi = 0, full_lo = INT32_MAX, full_hi = 0, all_lof = 0, all_uf = INT32_MAX;
+  int min_lof = INT32_MAX, max_uf = 0, max_lof = 0, min_uf = INT32_MAX;
+  int smin = INT32_MAX, smax = INT32_MIN, pmin = INT32_MAX, pmax = INT32_MIN;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int o = ot * kTile + lane + 32 * k;
+    valid[k] = o < a.outer_len;
+    rb[k] = load_bounds(a.mask, b, min(o, a.outer_len - 1));
+    seg[k] = KVAX_B200_PADDING_SEGMENT_ID; pos[k] = 0;
+    if (!valid[k]) continue;
+    if (kKvOuter) {
+      seg[k] = __ldg(a.tok.kv_seg + (long long)b * a.tok.kv_len + o);
+      pos[k] = a.tok.sequential ? o : __ldg(a.tok.kv_pos + (long long)b * a.tok.kv_len + o);
+    } else {
+      seg[k] = __ldg(a.tok.q_seg + (long long)b * a.tok.q_len + o);
+      pos[k] = query_position(a.tok, b, o);
+    }
+    if (rb[k].up > rb[k].lo) { vis_lo = min(vis_lo, rb[k].lo); vis_hi = max(vis_hi, rb[k].up); }
+    if (rb[k].uf > rb[k].lof) { full_lo = min(full_lo, rb[k].lof); full_hi = max(full_hi, rb[k].uf); }
+    min_lof = min(min_lof, rb[k].lo); max_lof = max(max_lof, rb[k].lof);
+    min_uf = min(min_uf, rb[k].uf); max_uf = max(max_uf, rb[k].up);
+    all_lof = max(all_lof, rb[k].lof); all_uf = min(all_uf, rb[k].uf);
+    smin = min(smin, seg[k]); smax = max(smax, seg[k]); pmin = min(pmin, pos[k]); pmax = max(pmax, pos[k]);
+  }
+  constexpr uint32_t kAll = 0xffffffffu;
+  vis_lo = __reduce_min_sync(kAll, vis_lo); vis_hi = __reduce_max_sync(kAll, vis_hi);
+  full_lo = __reduce_min_sync(kAll, full_lo); full_hi = __reduce_max_sync(kAll, full_hi);      // in the full range of some row
+  all_lof = __reduce_max_sync(kAll, all_lof); all_uf = min(__reduce_min_sync(kAll, all_uf), a.inner_len);   // ... of every row
+  const int left_lo = __reduce_min_sync(kAll, min_lof), left_hi = __reduce_max_sync(kAll, max_lof);   // union of the left ranges
+  const int right_lo = __reduce_min_sync(kAll, min_uf), right_hi = __reduce_max_sync(kAll, max_uf);   // union of the right ranges
+  smin = __reduce_min_sync(kAll, smin); smax = __reduce_max_sync(kAll, smax);
+  pmin = __reduce_min_sync(kAll, pmin); pmax = __reduce_max_sync(kAll, pmax);
+  vis_hi = min(vis_hi, a.n_inner_tiles * kTile);
+  // Rows beyond the end of the outer side: a query row is never stored, so it may see anything; a kv row must not
+  // (its P would be 2^-LSE, which can overflow, and is multiplied by the zero rows of K in dQ).
+  if (kKvOuter && (ot + 1) * kTile > a.outer_len) all_uf = 0;
+
+  // Exact element mask of one inner tile (whole warp): list entry of the tile, or kDropped.
+  auto exact = [&](int tile) -> uint32_t {
+    const int c0 = tile * kTile, lim = min(kTile, a.inner_len - c0);
+    const int4 s = __ldg(a.inner_summary + (long long)b * a.n_inner_tiles + tile);      // {smin, smax, pmin, pmax}
+    bool pass = false;                        // some row of this lane may hold an allowed element
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c1 = c0 + kTile;
+      const bool in_full = (c0 < rb[k].uf) && (c1 > rb[k].lof) && (rb[k].uf > rb[k].lof);
+      const bool seg_in = (s.x <= seg[k]) && (seg[k] <= s.y);
+      const bool left_ov = (c0 < rb[k].lof) && (c1 > rb[k].lo);
+      const bool right_ov = (c0 < rb[k].up) && (c1 > rb[k].uf);
+      const bool causal_ok = kKvOuter ? (s.w >= pos[k]) : (pos[k] >= s.z);
+      const bool cls = kKvOuter ? (right_ov || (left_ov && causal_ok)) : (left_ov || (right_ov && causal_ok));
+      pass = pass || (valid[k] && (in_full || (seg_in && cls)));
+    }
+    if (!__any_sync(kAll, pass)) return kDropped;
+    // this lane's four inner tokens; bit i of `starts`: token 4 lane + i starts a run
+    const int t0 = 4 * lane;
+    int ts[4], tp[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool in = t0 + i < lim;
+      ts[i] = in ? __ldg(inner_seg + c0 + t0 + i) : 0;
+      tp[i] = in ? inner_pos(c0 + t0 + i) : 0;
+    }
+    const int prev_s = __shfl_up_sync(kAll, ts[3], 1), prev_p = __shfl_up_sync(kAll, tp[3], 1);
+    uint32_t starts = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ps = i ? ts[i - 1] : prev_s, pp = i ? tp[i - 1] : prev_p;
+      const bool joined = (t0 + i > 0) && ts[i] == ps && pp != INT32_MAX && tp[i] == pp + 1;
+      starts |= (t0 + i < lim && !joined ? 1u : 0u) << i;
+    }
+    const int n_runs = __reduce_add_sync(kAll, __popc(starts));
+    uint32_t w[4][4] = {};
+    if (n_runs <= kMaxRuns) {
+      uint32_t word = starts << (4 * (lane & 7));           // starts of the 32 tokens of this group of eight lanes
+      word |= __shfl_xor_sync(kAll, word, 1); word |= __shfl_xor_sync(kAll, word, 2); word |= __shfl_xor_sync(kAll, word, 4);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (rb[k].uf > rb[k].lof) add_range(w[k], max(rb[k].lof - c0, 0), min(rb[k].uf - c0, lim));   // full: no condition
+      int next = 0;
+      while (next < lim) {
+        const int from = next;                              // run [from, next): segment `rs`, positions rp, rp + 1, ...
+        int q = (from + 1) >> 5;
+        next = lim;
+        uint32_t bits = q < 4 ? (__shfl_sync(kAll, word, (q & 3) * 8) & (kAll << ((from + 1) & 31))) : 0u;
+        while (q < 4) {
+          if (bits) { next = 32 * q + __ffs(bits) - 1; break; }
+          if (++q < 4) bits = __shfl_sync(kAll, word, q * 8);
+        }
+        const int sel = from & 3;
+        const int rs = __shfl_sync(kAll, sel == 0 ? ts[0] : (sel == 1 ? ts[1] : (sel == 2 ? ts[2] : ts[3])), from >> 2);
+        const int rp = __shfl_sync(kAll, sel == 0 ? tp[0] : (sel == 1 ? tp[1] : (sel == 2 ? tp[2] : tp[3])), from >> 2);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (seg[k] != rs) continue;
+          // causal part of the run: a prefix for a query row (position >= that of the token), a suffix for a kv row
+          int l0 = from, l1 = next, r0 = from, r1 = next;
+          if (kKvOuter) l0 = from + (pos[k] > rp ? int(min(uint32_t(pos[k]) - uint32_t(rp), uint32_t(kTile))) : 0);
+          else r1 = min(next, from + (pos[k] >= rp ? int(min(uint32_t(pos[k]) - uint32_t(rp), uint32_t(kTile))) + 1 : 0));
+          add_range(w[k], max(l0, rb[k].lo - c0), min(l1, rb[k].lof - c0));
+          add_range(w[k], max(r0, rb[k].uf - c0), min(r1, rb[k].up - c0));
+        }
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint4 x = row_mask_by_token<kKvOuter>(&a, rb[k], b, valid[k], seg[k], pos[k], c0);
+        w[k][0] = x.x; w[k][1] = x.y; w[k][2] = x.z; w[k][3] = x.w;
+      }
+    }
+    bool any = false, all = lim == kTile;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (!valid[k]) {
+        const uint32_t fill = kKvOuter ? 0u : kAll;
+        w[k][0] = w[k][1] = w[k][2] = w[k][3] = fill;
+      } else {
+        any = any || ((w[k][0] | w[k][1] | w[k][2] | w[k][3]) != 0u);
+      }
+      all = all && ((w[k][0] & w[k][1] & w[k][2] & w[k][3]) == kAll);
+    }
+    if (!__any_sync(kAll, any)) return kDropped;
+    if (__all_sync(kAll, all)) return uint32_t(tile);
+    uint32_t e = uint32_t(tile) | kPartialBit;
+    if (a.bitmaps) {
+      int slot = 0;
+      if (lane == 0) slot = atomicAdd(a.counters, 1);
+      slot = __shfl_sync(kAll, slot, 0);
+      if (slot < a.n_bitmaps) {
+        e |= kBitmapBit | (uint32_t(slot) << a.tile_bits);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          a.bitmaps[(long long)slot * kTile + lane + 32 * k] = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
+      }
+    }
+    return e;
+  };
+
+  uint32_t* out = a.tiles + ((long long)b * a.n_outer_tiles + ot) * a.n_inner_tiles;
+  int total = 0;
+  if (vis_hi > vis_lo) {
+    const int it0 = max(vis_lo, 0) / kTile;
+    const int it1 = min((vis_hi + kTile - 1) / kTile, a.n_inner_tiles);
+    for (int base = it0; base < it1; base += kChunk) {
+      const int n = min(kChunk, it1 - base);
+      if (tid == 0) s_n_cand = 0;
+      __syncthreads();
+      // A: interval test of this thread's inner tile
+      uint32_t entry = kDropped;
+      bool cand = false;
+      if (tid < n) {
+        const int c0 = (base + tid) * kTile, c1 = c0 + kTile;
+        if (all_lof <= c0 && c1 <= all_uf) {
+          entry = uint32_t(base + tid);
+        } else {
+          const int4 s = __ldg(a.inner_summary + (long long)b * a.n_inner_tiles + base + tid);
+          const bool seg_ov = (s.x <= smax) && (smin <= s.y);
+          const bool causal = kKvOuter ? (s.w >= pmin) : (pmax >= s.z);
+          const bool left_ov = (c0 < left_hi) && (c1 > left_lo), right_ov = (c0 < right_hi) && (c1 > right_lo);
+          const bool cls = kKvOuter ? (right_ov || (left_ov && causal)) : (left_ov || (right_ov && causal));
+          cand = ((c0 < full_hi) && (c1 > full_lo)) || (seg_ov && cls);
+        }
+        s_entry[tid] = entry;
+      }
+      const uint32_t m = __ballot_sync(kAll, cand);
+      int at = 0;
+      if (lane == 0 && m) at = atomicAdd(&s_n_cand, __popc(m));
+      at = __shfl_sync(kAll, at, 0);
+      if (cand) s_cand[at + __popc(m & ((1u << lane) - 1))] = tid;
+      __syncthreads();
+      // B: exact masks, one warp per tile
+      for (int i = warp; i < s_n_cand; i += kWarps) {
+        const int t = s_cand[i];
+        const uint32_t e = exact(base + t);
+        if (lane == 0) s_entry[t] = e;
+      }
+      __syncthreads();
+      // C: ordered compaction
+      entry = tid < n ? s_entry[tid] : kDropped;
+      const uint32_t kept = __ballot_sync(kAll, entry != kDropped);
+      if (lane == 0) s_warp_count[warp] = __popc(kept);
+      __syncthreads();
+      int before = total;
+#pragma unroll
+      for (int i = 0; i < kWarps; ++i) {
+        const int c = s_warp_count[i];
+        before += i < warp ? c : 0;
+        total += c;
+      }
+      if (entry != kDropped) out[before + __popc(kept & ((1u << lane) - 1))] = entry;
+      __syncthreads();
+    }
+  }
+  if (tid == 0) {
+    a.counts[(long long)b * a.n_outer_tiles + ot] = total;
+    __threadfence();
+    s_last = atomicAdd(a.counters + 1, 1) == int(gridDim.x * gridDim.y) - 1;
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    launch_order(s_order, a.counts, a.order, a.pair_order, a.n_outer_tiles, gridDim.y);
   }
 }
 
 }  // namespace
 
-void launch_tile_summaries(const TokenInfo& tok, int batch, int4* q_sum, int4* kv_sum, cudaStream_t s) {
+void launch_tile_summaries(const TokenInfo& tok, int batch, int4* q_sum, int4* kv_sum, int32_t* counters, cudaStream_t s) {
   const int nq = (tok.q_len + kTile - 1) / kTile, nk = (tok.kv_len + kTile - 1) / kTile;
   const long long warps = (long long)batch * (nq + nk);
-  tile_summary_kernel<<<int((warps + 7) / 8), 256, 0, s>>>(tok, q_sum, kv_sum, nq, nk, batch);
+  tile_summary_kernel<<<int((warps + 7) / 8), 256, 0, s>>>(tok, q_sum, kv_sum, nq, nk, batch, counters);
 }
 
 void launch_schedule(bool kv_outer, const ScheduleArgs& a, int batch, cudaStream_t s) {
   dim3 grid(a.n_outer_tiles, batch);
-  if (kv_outer) schedule_kernel<true><<<grid, kTile, 0, s>>>(a);
-  else schedule_kernel<false><<<grid, kTile, 0, s>>>(a);
-  order_kernel<<<1, 1024, 0, s>>>(a.counts, a.order, a.pair_order, a.n_outer_tiles, batch);
+  if (kv_outer) schedule_kernel<true><<<grid, kThreads, 0, s>>>(a);
+  else schedule_kernel<false><<<grid, kThreads, 0, s>>>(a);
 }
 
 }  // namespace kvx
