@@ -254,8 +254,8 @@ int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* workspace, size
  *     the workspace with bulk reduce-adds (the order of those fp32 additions varies from run
  *     to run, so dq is reproducible to rounding, not bit for bit) and a last kernel scales
  *     and casts it;
- *   two-kernel (KVAX_B200_BWD_TWO_KERNEL in `flags`, and every head_dim the fused kernel does
- *     not cover): a query-outer dQ kernel and a kv-outer dK/dV kernel, seven products per
+ *   two-kernel (KVAX_B200_BWD_TWO_KERNEL in `flags`):
+ *     a query-outer dQ kernel and a kv-outer dK/dV kernel, seven products per
  *     tile pair, bit-reproducible. */
 enum {
   KVAX_B200_BWD_TWO_KERNEL = 1,

@@ -77,21 +77,36 @@ constexpr int kThreads = (kMmaWarp + 1) * 32;          // 448
 constexpr int kSlice = kTile / 2;                      // columns per register-math thread
 constexpr int kStageBuf = 32 * 32 * 4;                 // one drain staging buffer: 32 rows x 32 fp32
 
-enum FBar { F_XFULL = 0, F_QFULL0, F_QFULL1, F_QEMPTY0, F_QEMPTY1, F_DOFULL, F_DOEMPTY, F_SFULL, F_PFULL, F_DPFULL,
-            F_DSFULL, F_DQFULL, F_DRAINED, F_ACCFULL, F_COUNT };
+enum FBar { F_XFULL = 0, F_QFULL0, F_QFULL1, F_QFULL2, F_QEMPTY0, F_QEMPTY1, F_QEMPTY2, F_DOFULL0, F_DOFULL1, F_DOEMPTY0,
+            F_DOEMPTY1, F_SFULL, F_PFULL, F_DPFULL, F_DSFULL, F_DQFULL0, F_DQFULL1, F_DRAINED0, F_DRAINED1, F_ACCFULL, F_COUNT };
+
+// Position in a ring of N buffers, and the parity of the barrier phase its present use belongs to.
+template <int N>
+struct Ring {
+  int st = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next() {
+    if (++st == N) { st = 0; ph ^= 1u; }
+  }
+};
 
 template <int D>
 struct FusedSmem {
   static constexpr int kTileBytes = kTile * D * 2;
   static constexpr int kBoxBytes = kTile * 64 * 2;
+  // head_dim 128 fills shared memory and TMEM; head_dim 64 has room for one more Q and dO tile, a second dS^T tile and, in
+  // TMEM, for two dQ tiles of their own (beside T2)
+  static constexpr int kQStages = D == 64 ? 3 : 2, kDoStages = D == 64 ? 2 : 1, kDsTiles = D == 64 ? 2 : 1;
+  static constexpr bool kOwnDq = D == 64;
   static constexpr int kX1 = 0, kX2 = kTileBytes;
   static constexpr int kQ = 2 * kTileBytes;                       // Q stage s at kQ + s * tile
-  static constexpr int kDO = 4 * kTileBytes;                      // dO, single buffer
-  static constexpr int kDS = 5 * kTileBytes;                      // dS^T tile: 128 kv rows x 128 queries bf16 (two boxes)
-  static constexpr int kStage = kDS + kTile * kTile * 2;          // drain warp w, buffer u: kStage + (2 w + u) * kStageBuf
+  static constexpr int kDO = kQ + kQStages * kTileBytes;          // dO stage s
+  static constexpr int kDsBytes = kTile * kTile * 2;              // dS^T tile: 128 kv rows x 128 queries (two boxes)
+  static constexpr int kDS = kDO + kDoStages * kTileBytes;
+  static constexpr int kStage = kDS + kDsTiles * kDsBytes;        // drain warp w, buffer u: kStage + (2 w + u) * kStageBuf
   static constexpr int kCols = kStage + kDrainWarps * 2 * kStageBuf;   // Q stage s: lse2[128] | delta[128]
   static constexpr int kColBytes = kTile * 4;
-  static constexpr int kBars = kCols + 2 * 2 * kColBytes;
+  static constexpr int kBars = kCols + kQStages * 2 * kColBytes;
   static constexpr int kTmemSlot = kBars + 8 * F_COUNT;
   static constexpr int kAbort = kTmemSlot + 4;
   static constexpr int kTotal = kAbort + 4;
@@ -176,7 +191,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
 
   if (tid == 0) {
     for (int i = 0; i < F_COUNT; ++i) {
-      const int n = (i == F_PFULL || i == F_DSFULL) ? kComputeThreads : (i == F_DRAINED ? kDrainWarps * 32 : 1);
+      const int n = (i == F_PFULL || i == F_DSFULL) ? kComputeThreads : ((i == F_DRAINED0 || i == F_DRAINED1) ? kDrainWarps * 32 : 1);
       mbar_init(&bars[i], n);
     }
     *abort_flag = 0;
@@ -189,6 +204,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tT1 = tmem_base, tT2 = tmem_base + kTile;
   const uint32_t tDV = tmem_base + 2 * kTile, tDK = tmem_base + 2 * kTile + D;
+  // dQ of item i: over dP^T in T2, or columns of its own, taken in turn
+  auto dq_columns = [&](int i) { return L::kOwnDq ? tDK + D + (i & 1) * D : tT2; };
 
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ producer (whole warp; one elected lane issues)
@@ -207,17 +224,19 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     bool ok = true;
     uint32_t e_next = __ldg(list);                 // list entries are fetched one iteration ahead
     int li = 0, qh = first_head;                  // index into the list, query head
+    Ring<L::kQStages> rq;
+    Ring<L::kDoStages> rd;
     PH_BEGIN()
     for (int i = 0; i < n && ok; ++i) {
-      const int st = i & 1;
+      const int st = rq.st;
       const int u = int(e_next & a.list.tile_mask);
       const int yh = qh;
       if (++li == cnt) { li = 0; ++qh; }
       if (i + 1 < n) e_next = __ldg(list + li);
       PH(1)
-      // ---- Q(i) with LSE2 / delta: its stage is free once dK(i-2) has completed
-      if (i >= 2) {
-        ok = mbar_wait(&bars[F_QEMPTY0 + st], ((i >> 1) - 1) & 1, abort_flag, a.status, F_QEMPTY0 + st);
+      // ---- Q(i) with LSE2 / delta: its stage is free once dK of the item that had it before has completed
+      if (i >= L::kQStages) {
+        ok = mbar_wait(&bars[F_QEMPTY0 + st], rq.ph ^ 1u, abort_flag, a.status, F_QEMPTY0 + st);
         ok = __all_sync(0xffffffffu, ok);
       }
       PH(0)
@@ -250,20 +269,22 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         }
       }
       __syncwarp();
-      // ---- dO(i): the single buffer is free once dV(i-1) has completed
-      if (i >= 1) {
-        ok = mbar_wait(&bars[F_DOEMPTY], uint32_t((i - 1) & 1), abort_flag, a.status, F_DOEMPTY);
+      // ---- dO(i): its buffer is free once dV of the item that had it before has completed
+      if (i >= L::kDoStages) {
+        ok = mbar_wait(&bars[F_DOEMPTY0 + rd.st], rd.ph ^ 1u, abort_flag, a.status, F_DOEMPTY0 + rd.st);
         ok = __all_sync(0xffffffffu, ok);
       }
       PH(2)
       if (!ok) break;
       if (elect_one()) {
-        mbar_arrive_expect_tx(&bars[F_DOFULL], L::kTileBytes);
+        mbar_arrive_expect_tx(&bars[F_DOFULL0 + rd.st], L::kTileBytes);
 #pragma unroll
         for (int x = 0; x < D / 64; ++x)
-          tma_load_4d(smem + L::kDO + x * L::kBoxBytes, &tmap_do, &bars[F_DOFULL], x * 64, yh, u * kTile, b);
+          tma_load_4d(smem + L::kDO + rd.st * L::kTileBytes + x * L::kBoxBytes, &tmap_do, &bars[F_DOFULL0 + rd.st], x * 64, yh, u * kTile, b);
       }
       __syncwarp();
+      rq.next();
+      rd.next();
     }
     PH_END(3, n)
   } else if (warp == kMmaWarp) {
@@ -278,7 +299,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     const uint32_t do_k_lo = sdesc_lo_sw128(smem_u32(smem + L::kDO), 16);            // dO, head dimension contracted (dP^T)
     const uint32_t do_n_lo = sdesc_lo_sw128(smem_u32(smem + L::kDO), L::kBoxBytes);  // dO, queries contracted (dV)
     const uint32_t ds_addr = smem_u32(smem + L::kDS);
-    const uint32_t ds_mn_lo = sdesc_lo_sw128(ds_addr, L::kBoxBytes), ds_k_lo = sdesc_lo_sw128(ds_addr, 16);
+    const uint32_t ds_mn_lo0 = sdesc_lo_sw128(ds_addr, L::kBoxBytes), ds_k_lo0 = sdesc_lo_sw128(ds_addr, 16);
+    constexpr uint32_t kTileStep = L::kTileBytes >> 4, kDsStep = L::kDsBytes >> 4;   // descriptor steps between buffers
     const int n = __shfl_sync(0xffffffffu, n_items, 0);
     bool ok = true;
     // `tmem_sync`: the barrier orders TMEM loads / stores of other threads before the MMAs that follow; barriers
@@ -297,7 +319,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     };
     wait(F_XFULL, 0, false);
     if (ok) wait(F_QFULL0, 0, false);
-    if (ok) wait(F_DOFULL, 0, false);
+    if (ok) wait(F_DOFULL0, 0, false);
     if (ok) {
       if (elect_one()) {
         issue_t(tT1, x1_lo, sdesc_lo_sw128(qbase, 16));
@@ -307,11 +329,23 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       }
       __syncwarp();
     }
+    Ring<L::kQStages> rq, rqn;                   // buffers of Q(i), Q(i+1)
+    Ring<L::kDoStages> rd, rdn;
+    rqn.next();
+    rdn.next();
+    auto issue_dp_next = [&]() {                 // dP^T of item i+1
+      wait(F_DOFULL0 + rdn.st, rdn.ph, false);
+      if (!ok) return;
+      if (elect_one()) {
+        issue_t(tT2, x2_lo, do_k_lo + rdn.st * kTileStep);
+        umma_commit(&bars[F_DPFULL]);
+      }
+      __syncwarp();
+    };
     PH_BEGIN()
     for (int i = 0; i < n && ok; ++i) {
-      const int st = i & 1;
       const uint32_t ph = uint32_t(i & 1);
-      const uint32_t yq = qbase + st * L::kTileBytes, yqn = qbase + (st ^ 1) * L::kTileBytes;
+      const uint32_t yq = qbase + rq.st * L::kTileBytes, yqn = qbase + rqn.st * L::kTileBytes;
       const uint32_t acc_on = (i > 0) ? 1u : 0u;
       const bool more = (i + 1 < n);
       wait(F_PFULL, ph, true);                                                      // P^T(i) written, S^T(i) consumed
@@ -319,15 +353,16 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       if (!ok) break;
       if (elect_one()) {
         // dV += P^T dO: the half h of the register-math threads wrote its four K-steps at column offset 64 h
+        const uint32_t do_lo = do_n_lo + rd.st * kTileStep;
 #pragma unroll
         for (int kk = 0; kk < kTile / 16; ++kk)
-          umma_ts_lo(tDV, tT1 + (kk >> 2) * kSlice + (kk & 3) * 8, do_n_lo + ((kk * 16 * 128) >> 4), idesc_dv, acc_on | (kk > 0));
-        umma_commit(&bars[F_DOEMPTY]);                                              // dO(i) is dead: its buffer may take dO(i+1)
+          umma_ts_lo(tDV, tT1 + (kk >> 2) * kSlice + (kk & 3) * 8, do_lo + ((kk * 16 * 128) >> 4), idesc_dv, acc_on | (kk > 0));
+        umma_commit(&bars[F_DOEMPTY0 + rd.st]);                                     // dO(i) is dead: its buffer may be refilled
       }
       __syncwarp();
       PH(1)
       if (more) {
-        wait(F_QFULL0 + (st ^ 1), ((i + 1) >> 1) & 1, false);
+        wait(F_QFULL0 + rqn.st, rqn.ph, false);
         PH(2)
         if (!ok) break;
         if (elect_one()) {
@@ -340,13 +375,20 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       wait(F_DSFULL, ph, true);                                                     // dS^T(i) in its tile, dP^T(i) consumed
       PH(4)
       if (!ok) break;
+      const uint32_t tdq = dq_columns(i);
+      if (L::kOwnDq) {
+        if (more) issue_dp_next();                                                  // T2 is free already
+        if (ok && i >= 2) wait(F_DRAINED0 + (i & 1), uint32_t((i >> 1) - 1) & 1u, true);   // dQ(i-2) has left its columns
+        if (!ok) break;
+      }
       if (elect_one()) {
-        // dQ(i) = dS K over the dP^T columns: both operands read with kv as the contraction index (16 kv rows per
-        // step = 16 lines of 128 bytes)
+        const uint32_t ds_off = L::kDsTiles == 2 ? (i & 1) * kDsStep : 0u;
+        const uint32_t ds_mn_lo = ds_mn_lo0 + ds_off, ds_k_lo = ds_k_lo0 + ds_off;
+        // dQ(i) = dS K: both operands read with kv as the contraction index (16 kv rows per step = 16 lines of 128 bytes)
 #pragma unroll
         for (int kk = 0; kk < kTile / 16; ++kk)
-          umma_ss_lo(tT2, ds_mn_lo + ((kk * 16 * 128) >> 4), kmn_lo + ((kk * 16 * 128) >> 4), idesc_dq, kk > 0);
-        umma_commit(&bars[F_DQFULL]);
+          umma_ss_lo(tdq, ds_mn_lo + ((kk * 16 * 128) >> 4), kmn_lo + ((kk * 16 * 128) >> 4), idesc_dq, kk > 0);
+        umma_commit(&bars[F_DQFULL0 + (L::kOwnDq ? (i & 1) : 0)]);
         // dK(i) += dS^T(i) Q(i)
         const uint32_t q_lo = sdesc_lo_sw128(yq, L::kBoxBytes);
 #pragma unroll
@@ -354,23 +396,19 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
           const uint32_t off = ((kk >> 2) * L::kBoxBytes + (kk & 3) * 32) >> 4;
           umma_ss_lo(tDK, ds_k_lo + off, q_lo + ((kk * 16 * 128) >> 4), idesc_dk, acc_on | (kk > 0));
         }
-        umma_commit(&bars[F_QEMPTY0 + st]);                                         // Q(i) is dead; also: the dS^T tile may be rewritten
+        umma_commit(&bars[F_QEMPTY0 + rq.st]);                                      // Q(i) is dead; also: the dS^T tile may be rewritten
         if (!more) umma_commit(&bars[F_ACCFULL]);
       }
       __syncwarp();
       PH(5)
-      if (more) {
-        wait(F_DRAINED, ph, true);                                                  // dQ(i) has left the T2 columns
+      if (!L::kOwnDq && more) {
+        wait(F_DRAINED0, ph, true);                                                 // dQ(i) has left the T2 columns
         PH(6)
-        if (ok) wait(F_DOFULL, uint32_t((i + 1) & 1), false);
+        if (ok) issue_dp_next();
         if (!ok) break;
-        if (elect_one()) {
-          issue_t(tT2, x2_lo, do_k_lo);                                             // dP^T of item i+1
-          umma_commit(&bars[F_DPFULL]);
-        }
-        __syncwarp();
         PH(7)
       }
+      rq.next(); rqn.next(); rd.next(); rdn.next();
     }
     PH_END(1, n)
   } else if (is_compute) {
@@ -395,14 +433,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     // awaited), so that their global loads never sit in front of the exponentials
     uint32_t keep_next[2] = {0xffffffffu, 0xffffffffu};
     if (e_next & kPartialBit) item_keep(e_next, keep_next);
-    uint8_t* ds_row = smem + L::kDS + half * L::kBoxBytes + row * 128;   // this thread's 128-byte row of the dS^T tile
+    uint8_t* ds_row = smem + L::kDS + half * (kTile * 128) + row * 128;  // this thread's 128-byte row of the dS^T tile
+    Ring<L::kQStages> rq, rfree;                            // buffer of Q(i); of the last item that read the tile dS^T(i) goes to
     PH_BEGIN()
     for (int i = 0; i < n_items && ok; ++i) {
       const uint32_t e = e_next;
       if (++li == count) li = 0;
       if (i + 1 < n_items) e_next = ldg_pinned(list + li);
       const bool partial = (e & kPartialBit) != 0;
-      const int st = i & 1;
+      const int st = rq.st;
       const uint32_t ph = uint32_t(i & 1);
       const float* cs = s_cols + st * 2 * kTile;
       const float4* cs_lse = reinterpret_cast<const float4*>(cs + cb);
@@ -410,7 +449,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       const uint32_t keep[2] = {keep_next[0], keep_next[1]};
 
       // LSE2 / delta of this item have landed together with its Q tile
-      ok = mbar_wait(&bars[F_QFULL0 + st], (i >> 1) & 1, abort_flag, a.status, F_QFULL0 + st);
+      ok = mbar_wait(&bars[F_QFULL0 + st], rq.ph, abort_flag, a.status, F_QFULL0 + st);
+      rq.next();
       PH(1)
       if (!ok) break;
 
@@ -457,15 +497,16 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       tc_fence_after();
       uint32_t dp[2][16];                                     // 16 columns at a time, the next request in flight
       tmem_ld16(my_t2, dp[0]);
-      if (i > 0) {      // dQ(i-1) and dK(i-1), the readers of the tile, have completed (the commit that frees Q stage (i-1) & 1)
-        ok = mbar_wait(&bars[F_QEMPTY0 + ((i - 1) & 1)], ((i - 1) >> 1) & 1, abort_flag, a.status, F_QEMPTY0 + ((i - 1) & 1));
+      if (i >= L::kDsTiles) {      // dQ and dK of the tile's last item have completed (the commit that frees that item's Q stage)
+        ok = mbar_wait(&bars[F_QEMPTY0 + rfree.st], rfree.ph, abort_flag, a.status, F_QEMPTY0 + rfree.st);
+        rfree.next();
         if (!ok) break;
       }
       PH(5)
       {
         // kv row `row`, queries [64 half, 64 half + 64) = one 128-byte row of box `half`: eight 16-byte chunks at the
         // positions the 128-byte swizzle assigns them
-        uint8_t* slot = ds_row;
+        uint8_t* slot = ds_row + (L::kDsTiles == 2 ? (i & 1) * L::kDsBytes : 0);
 #pragma unroll
         for (int sc = 0; sc < 4; ++sc) {                      // columns [16 sc, 16 sc + 16) of this thread's 64
           if (sc + 1 < 4) tmem_ld16(my_t2 + (sc + 1) * 16, dp[(sc + 1) & 1]);
@@ -557,7 +598,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       if (++li == count) { li = 0; ++qh; }
       if (i + 1 < n_items) e_next = ldg_pinned(list + li);
       const bool live = q0 < q_len;                           // rows beyond the sequence are clipped by TMA; skip all-out boxes
-      ok = mbar_wait(&bars[F_DQFULL], uint32_t(i & 1), abort_flag, a.status, F_DQFULL);
+      const int db = L::kOwnDq ? (i & 1) : 0;
+      const uint32_t tdq = dq_columns(i) + lane_base;
+      ok = mbar_wait(&bars[F_DQFULL0 + db], uint32_t(L::kOwnDq ? (i >> 1) : i) & 1u, abort_flag, a.status, F_DQFULL0 + db);
       PH(0)
       if (!ok) break;
       tc_fence_after();
@@ -585,25 +628,36 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         if (lane == 0) bulk_wait_group_read<1>();
         __syncwarp();
       };
-      static_assert(D == 128, "drain schedule written for four 32-column chunks");
-      uint32_t x0[32], x1[32], x2[32];
-      tmem_ld32(tT2 + lane_base, x0);
-      tmem_ld32(tT2 + lane_base + 32, x1);
-      tmem_ld32(tT2 + lane_base + 64, x2);
-      buffer_free();                                          // buffer 0: chunk 2 of the previous item, long gone
-      tmem_ld_wait(x0);
-      put(0, x0);
-      tmem_ld32(tT2 + lane_base + 96, x0);                    // chunk 3 takes the registers of chunk 0
-      tmem_ld_wait(x1);
-      tmem_ld_wait(x2);
-      tmem_ld_wait(x0);
-      tc_fence_before();
-      mbar_arrive(&bars[F_DRAINED]);                          // the T2 columns may take dP^T(i+1)
-      PH(1)
-      reduce(0);
-      buffer_free(); put(1, x1); reduce(1);
-      buffer_free(); put(2, x2); reduce(2);
-      buffer_free(); put(3, x0); reduce(3);
+      uint32_t x0[32], x1[32];
+      tmem_ld32(tdq, x0);
+      tmem_ld32(tdq + 32, x1);
+      if constexpr (D == 128) {
+        uint32_t x2[32];
+        tmem_ld32(tdq + 64, x2);
+        buffer_free();                                        // buffer 0: chunk 2 of the previous item, long gone
+        tmem_ld_wait(x0);
+        put(0, x0);
+        tmem_ld32(tdq + 96, x0);                              // chunk 3 takes the registers of chunk 0
+        tmem_ld_wait(x1);
+        tmem_ld_wait(x2);
+        tmem_ld_wait(x0);
+        tc_fence_before();
+        mbar_arrive(&bars[F_DRAINED0]);                       // the T2 columns may take dP^T(i+1)
+        PH(1)
+        reduce(0);
+        buffer_free(); put(1, x1); reduce(1);
+        buffer_free(); put(2, x2); reduce(2);
+        buffer_free(); put(3, x0); reduce(3);
+      } else {
+        static_assert(D == 64 || D == 128, "two or four 32-column chunks");
+        tmem_ld_wait(x0);
+        tmem_ld_wait(x1);
+        tc_fence_before();
+        mbar_arrive(&bars[F_DRAINED0 + db]);                  // these columns may take dQ(i+2)
+        PH(1)
+        buffer_free(); put(0, x0); reduce(0);
+        buffer_free(); put(1, x1); reduce(1);
+      }
       PH(2)
     }
     if (dw == 0) { PH_END(2, n_items) }
@@ -649,7 +703,6 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_cast_kernel(const float* __re
 
 template <int D, bool kF16>
 int launch_fused(const FusedBwdLaunch& L, cudaStream_t stream) {
-  static_assert(D == 128, "the drain is written for four 32-column chunks");
   constexpr int smem = FusedSmem<D>::kTotal;
   auto kern = attn_bwd_fused_kernel<D, kF16>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return KVAX_B200_ELAUNCH;
@@ -660,7 +713,7 @@ int launch_fused(const FusedBwdLaunch& L, cudaStream_t stream) {
 
 }  // namespace
 
-bool attn_bwd_fused_supports(int head_dim) { return head_dim == 128; }
+bool attn_bwd_fused_supports(int head_dim) { return head_dim == 64 || head_dim == 128; }
 
 #ifdef KVAX_PHASE_CLOCKS
 // profiling builds only: where the phase clocks go ((grid, 4, 12) uint32 in device memory), or null
@@ -671,6 +724,7 @@ extern "C" int kvax_b200_debug_set_phase_buffer(unsigned int* buf) {
 
 int launch_attn_bwd_fused(const FusedBwdLaunch& L, cudaStream_t stream) {
   if (L.head_dim == 128) return L.dtype == KVAX_B200_F16 ? launch_fused<128, true>(L, stream) : launch_fused<128, false>(L, stream);
+  if (L.head_dim == 64) return L.dtype == KVAX_B200_F16 ? launch_fused<64, true>(L, stream) : launch_fused<64, false>(L, stream);
   return KVAX_B200_EUNSUPPORTED;
 }
 
