@@ -235,7 +235,10 @@ typedef struct kvax_b200_attn_fwd_params {
 enum { KVAX_B200_FWD_ONE_TILE = 1, KVAX_B200_FWD_TILE_PAIRS = 2, KVAX_B200_FWD_HEAD_PAIRS = 4,
        /* query tiles without any key tile get lse = +inf instead of the reference's 0 (flash_attention_triton.py:253-258),
           so that kvax_b200_attn_merge can tell them from rows that have keys */
-       KVAX_B200_FWD_EMPTY_LSE_INF = 8 };
+       KVAX_B200_FWD_EMPTY_LSE_INF = 8,
+       /* the kv tiles of all query tiles divided evenly over the SMs, the query heads of a kv head in one tile where that
+          makes fewer tiles: what short queries on long keys get by default */
+       KVAX_B200_FWD_SPLIT = 16 };
 
 size_t kvax_b200_attn_fwd_workspace_bytes(const kvax_b200_attn_fwd_params* p);
 int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* workspace, size_t workspace_bytes,
@@ -249,7 +252,7 @@ int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* workspace, size
  * context-parallel reduction; dq is in the input dtype with its own strides.
  *
  * Two schedules produce the gradients:
- *   fused (default, head_dim 128): one kv-outer kernel computes dK, dV and dQ with five
+ *   fused (default, head_dim 64 and 128): one kv-outer kernel computes dK, dV and dQ with five
  *     matrix products per tile pair; partial dQ tiles are summed into an fp32 accumulator in
  *     the workspace with bulk reduce-adds (the order of those fp32 additions varies from run
  *     to run, so dq is reproducible to rounding, not bit for bit) and a last kernel scales

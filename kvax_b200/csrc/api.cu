@@ -34,13 +34,15 @@ EncodeTiledFn encode_tiled_fn() {
 
 // bf16 tensor (batch, seq, heads, D) with element strides {batch, seq, head}; boxes of
 // 128 rows x 64 columns of one head, 128-byte swizzle, out-of-range rows read as zero.
-int make_tmap(CUtensorMap* map, const void* base, int batch, int seq, int heads, int d, const int64_t* strides, int dtype) {
+// Query tiles of several heads: boxes of `box_seq` rows of `box_heads` heads each (row-major: token, head).
+int make_tmap(CUtensorMap* map, const void* base, int batch, int seq, int heads, int d, const int64_t* strides, int dtype,
+              int box_seq = kTile, int box_heads = 1) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return KVAX_B200_ENODEVICE;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || ((strides[0] | strides[1] | strides[2]) & 7)) return KVAX_B200_EUNSUPPORTED;
   cuuint64_t dims[4] = {cuuint64_t(d), cuuint64_t(heads), cuuint64_t(seq), cuuint64_t(batch)};
   cuuint64_t gstr[3] = {cuuint64_t(strides[2]) * 2, cuuint64_t(strides[1]) * 2, cuuint64_t(strides[0]) * 2};
-  cuuint32_t box[4] = {64, 1, cuuint32_t(kTile), 1};
+  cuuint32_t box[4] = {64, cuuint32_t(box_heads), cuuint32_t(box_seq), 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUtensorMapDataType elem = dtype == KVAX_B200_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUresult r = fn(map, elem, 4, const_cast<void*>(base), dims, gstr, box, estr,
@@ -130,6 +132,7 @@ void fill_schedule(ScheduleArgs* sa, const MaskView& mv, const TokenInfo& tok, c
   sa->counts = reinterpret_cast<int32_t*>(ws + ll.counts_off);
   sa->order = reinterpret_cast<int32_t*>(ws + ll.order_off);
   sa->pair_order = sa->order + size_t(ll.batch) * ll.n_outer;
+  sa->prefix = nullptr;
   sa->inner_summary = inner_summary;
   sa->counters = counters;
   sa->bitmaps = ll.n_bitmaps ? reinterpret_cast<uint4*>(ws + ll.bitmaps_off) : nullptr;
@@ -139,7 +142,7 @@ void fill_schedule(ScheduleArgs* sa, const MaskView& mv, const TokenInfo& tok, c
 }
 
 void fill_list(TileList* l, const ScheduleArgs& sa) {
-  l->tiles = sa.tiles; l->counts = sa.counts; l->order = sa.order; l->pair_order = sa.pair_order; l->bitmaps = sa.bitmaps;
+  l->tiles = sa.tiles; l->counts = sa.counts; l->order = sa.order; l->pair_order = sa.pair_order; l->prefix = sa.prefix; l->bitmaps = sa.bitmaps;
   l->tile_bits = sa.tile_bits; l->tile_mask = (1u << sa.tile_bits) - 1;
   l->n_outer_tiles = sa.n_outer_tiles; l->n_inner_tiles = sa.n_inner_tiles;
 }
@@ -166,10 +169,66 @@ extern "C" const char* kvax_b200_error_string(int code) {
   }
 }
 
+namespace {
+
+// How the split forward (attn_fwd_split.cu) cuts a call into query tiles, and whether it is the kernel to take.
+struct SplitPlan { bool use; int pack, tile_tokens, token_blocks, head_items, min_tiles; };
+
+SplitPlan split_plan(const kvax_b200_attn_fwd_params& p) {
+  const kvax_b200_attn_shape& s = p.shape;
+  const int group = s.q_heads / s.kv_heads, n_outer = cdiv(s.q_len, kTile), n_inner = cdiv(s.kv_len, kTile);
+  SplitPlan l{false, 1, kTile, 1, s.q_heads, kSplitMinTiles};
+  // The heads of a kv group share a query tile when that makes fewer of them: tokens of a tile are then the largest power of
+  // two (a tile must not cross a list's 128 tokens) whose rows fit.
+  if (group > 1 && group <= kTile && n_outer == 1) {
+    int t = kTile;
+    while (t * group > kTile) t /= 2;
+    if (cdiv(s.q_len, t) * s.kv_heads < s.q_heads) {
+      l.pack = group; l.tile_tokens = t; l.token_blocks = cdiv(s.q_len, t); l.head_items = s.kv_heads;
+    }
+  }
+  // The CTA that merges the parts of an item spends about three tiles' time per part when all 128 rows are in use: shares of
+  // sqrt(3 n) tiles balance the parts of a list of n tiles against the tiles of a part (1 x 32 tokens on 9000 keys, 32/8
+  // heads: 98 us with shares of four tiles, 68 with fifteen, one tile per CTA 76).
+  const int rows = (s.q_len < l.tile_tokens ? s.q_len : l.tile_tokens) * l.pack;
+  const int balanced = int(sqrtf(3.f * n_inner * rows / kTile));
+  if (balanced > l.min_tiles) l.min_tiles = balanced;
+  const long long items = (long long)s.batch * n_outer * l.token_blocks * l.head_items;
+  const bool fits = items * n_inner < (1ll << 30);           // tiles are counted in 32 bits
+  if (p.flags & KVAX_B200_FWD_SPLIT) l.use = fits;
+  else if (p.flags & (KVAX_B200_FWD_ONE_TILE | KVAX_B200_FWD_TILE_PAIRS | KVAX_B200_FWD_HEAD_PAIRS)) l.use = false;
+  else
+    // Measured (us of the attention kernel, one tile per CTA / split), bf16, 32/8 heads, one query token: 16 x 8k keys
+    // 230 / 76, 16 x 2k 79 / 30, 2 x 2k 19.9 / 19.6, 2 x 1k 14 / 18, 64 x 1k 171 / 55, 64 x 500 129 / 40: pays from 2k keys
+    // on, and on shorter ones where packing saves whole waves of CTAs.  Not packed it pays for few items on long lists only
+    // (16/16 heads, 2 x 4k: 30 / 18; 8/2 heads, 256 tokens on 32k: 244 / 101; 4/4 heads, 3 x 200 tokens on 4k: 39 / 41): a tile
+    // costs a quarter more than in the one-tile kernel, so 2 x 1000 tokens on 17k keys, 512 items, take 548 / 595, and short
+    // lists drown in partial results (1500 tokens of packed documents, 8/2 heads: 15 / 49), which queries that are not few
+    // against the keys can have.
+    l.use = fits && ((n_inner >= (n_outer > 1 ? 64 : 16) && n_inner >= 4 * n_outer && (l.pack > 1 || 2 * items <= kSplitCtas)) ||
+                     (l.pack > 1 && n_inner >= 4 && (long long)s.batch * s.q_heads >= 2 * kSplitCtas));
+  return l;
+}
+
+struct FwdLayout { ListLayout list; SummaryLayout sum; size_t parts_off, part_ml_off, total; SplitPlan split; };
+
+FwdLayout fwd_layout(const kvax_b200_attn_fwd_params& p) {
+  const kvax_b200_attn_shape& s = p.shape;
+  FwdLayout l;
+  l.split = split_plan(p);
+  l.list = list_layout(s.batch, s.q_len, s.kv_len, 0, true);
+  l.sum = summary_layout(s.batch, s.q_len, s.kv_len, l.list.total);
+  l.parts_off = l.sum.total;
+  l.part_ml_off = l.parts_off + (l.split.use ? align256(size_t(2 * kSplitCtas) * kTile * s.head_dim * sizeof(float)) : 0);
+  l.total = l.part_ml_off + (l.split.use ? align256(size_t(2 * kSplitCtas) * kTile * sizeof(float2)) : 0);
+  return l;
+}
+
+}  // namespace
+
 extern "C" size_t kvax_b200_attn_fwd_workspace_bytes(const kvax_b200_attn_fwd_params* p) {
   if (!p || check_shape(p->shape) != KVAX_B200_OK) return 0;
-  const ListLayout ll = list_layout(p->shape.batch, p->shape.q_len, p->shape.kv_len, 0, true);
-  return summary_layout(p->shape.batch, p->shape.q_len, p->shape.kv_len, ll.total).total;
+  return fwd_layout(*p).total;
 }
 
 extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* workspace, size_t workspace_bytes,
@@ -178,9 +237,10 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   const kvax_b200_attn_shape& s = p->shape;
   int rc = check_shape(s);
   if (rc) return rc;
-  const ListLayout ll = list_layout(s.batch, s.q_len, s.kv_len, 0, true);
-  const SummaryLayout sl = summary_layout(s.batch, s.q_len, s.kv_len, ll.total);
-  if (!workspace || workspace_bytes < sl.total || (reinterpret_cast<uintptr_t>(workspace) & 255)) return KVAX_B200_EWORKSPACE;
+  const FwdLayout fl = fwd_layout(*p);
+  const ListLayout& ll = fl.list;
+  const SummaryLayout& sl = fl.sum;
+  if (!workspace || workspace_bytes < fl.total || (reinterpret_cast<uintptr_t>(workspace) & 255)) return KVAX_B200_EWORKSPACE;
   if ((s.o_strides[0] | s.o_strides[1] | s.o_strides[2]) & 7 || (reinterpret_cast<uintptr_t>(p->out) & 15)) return KVAX_B200_EUNSUPPORTED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
@@ -194,6 +254,7 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   int4* kv_sum = reinterpret_cast<int4*>(ws + sl.kv_off);
   int32_t* counters = reinterpret_cast<int32_t*>(ws + sl.counters_off);
   fill_schedule(&sa, mv, token_info(s), ws, ll, kv_sum, counters, s.q_len, s.kv_len);
+  if (fl.split.use) sa.prefix = sa.order;       // the split kernel has no launch order; as many entries at least
   const int stages = p->stages ? p->stages : 3;
   if (stages & 1) {
     launch_tile_summaries(sa.tok, s.batch, q_sum, kv_sum, counters, st);
@@ -203,7 +264,9 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   if (!(stages & 2)) return KVAX_B200_OK;
 
   FwdLaunch L;
-  rc = make_tmap(&L.tmap_q, p->q, s.batch, s.q_len, s.q_heads, s.head_dim, s.q_strides, s.dtype);  if (rc) return rc;
+  rc = make_tmap(&L.tmap_q, p->q, s.batch, s.q_len, s.q_heads, s.head_dim, s.q_strides, s.dtype,
+                 fl.split.use ? fl.split.tile_tokens : kTile, fl.split.use ? fl.split.pack : 1);
+  if (rc) return rc;
   rc = make_tmap(&L.tmap_k, p->k, s.batch, s.kv_len, s.kv_heads, s.head_dim, s.k_strides, s.dtype); if (rc) return rc;
   rc = make_tmap(&L.tmap_v, p->v, s.batch, s.kv_len, s.kv_heads, s.head_dim, s.v_strides, s.dtype); if (rc) return rc;
   FwdArgs& a = L.args;
@@ -228,6 +291,11 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   a.pair_heads = (a.group % 2 == 0) ? 1 : 0;
   if (p->flags & KVAX_B200_FWD_TILE_PAIRS) a.pair_heads = 0;
   if ((p->flags & KVAX_B200_FWD_HEAD_PAIRS) && a.group % 2) return KVAX_B200_EUNSUPPORTED;
+  a.pack = fl.split.pack; a.tile_tokens = fl.split.tile_tokens; a.token_blocks = fl.split.token_blocks; a.head_items = fl.split.head_items;
+  a.min_tiles = fl.split.min_tiles;
+  a.parts = reinterpret_cast<float*>(ws + fl.parts_off); a.part_ml = reinterpret_cast<float2*>(ws + fl.part_ml_off);
+  a.part_counters = counters + 4;
+  if (fl.split.use) return launch_attn_fwd_split(L, st);
   return pairs ? launch_attn_fwd(L, st) : launch_attn_fwd_one(L, st);
 }
 

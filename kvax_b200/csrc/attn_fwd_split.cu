@@ -1,0 +1,602 @@
+// Flash-attention forward for sm_100a (B200), work split evenly over the SMs: the variant for calls with too few query
+// tiles to fill 148 SMs -- decoding, and chunks of a prompt on top of a long cache.
+//
+// One CTA per SM.  The kv tiles of all work items (query tile, head, batch) form one sequence; every CTA takes an equal
+// contiguous share of it, so a long list is divided over several CTAs and a CTA walks the end of one list, whole lists, and
+// the start of another ("segments").  A CTA that holds only part of an item writes that part (output relative to its
+// maximum, maximum, row sum; fp32) to the workspace; whoever finishes the item's last part merges them all: nobody waits
+// for another CTA.
+//
+// Packing: with few query tokens (q_len <= 128) and grouped-query attention the 128 rows of a query tile are the query
+// tokens times the `pack` = group heads that share a kv head (row = token * pack + head), loaded by TMA as a
+// (tokens x heads) box, so K and V are read once per kv head and not once per query head.  A softmax warp whose 32 rows hold
+// no query skips the arithmetic (its rows of P are whatever TMEM holds; rows of an MMA do not mix).
+//
+// What bounds it: decoding reads K and V once, 16 sequences of 4k-8k keys, 32/8 heads, head_dim 128: 400 MB = 62 us at
+// the measured copy rate; measured 76 us (5.3 TB/s), one tile per CTA 230 us (every query head reads them, lists of up to 64
+// tiles on 512 CTAs); 64 sequences 250 / 787 us, one sequence of 32k keys 33 / 194 us.
+//
+// Warps as in attn_fwd_one.cu: two softmax groups of four warps (even / odd tiles, merged at the end of a segment), the K
+// (and Q) producer, the MMA issuer, the V producer.  Rings and their phases run on across segments, so the K / V loads and
+// the first products of the next segment overlap the end of the current one; Q is double buffered for that.
+// TMEM (512 columns): S0 | S1 | O0 | O1.  Shared memory: Q 2 x 32 KB, K 3 x 32 KB, V 2 x 32 KB, exchange 2 KB.
+//
+// Semantics as attn_fwd_one.cu (kvax/ops/flash_attention_triton.py:137-370).
+#include "attn_common.cuh"
+#include "internal.h"
+#include "ptx.cuh"
+
+namespace kvx {
+
+namespace {
+
+constexpr int kSoftmaxThreads = 256;                 // two groups of 128
+constexpr int kKWarp = 8, kMmaWarp = 9, kVWarp = 10;
+constexpr int kThreads = 11 * 32;
+constexpr int kTmemCols = 512;
+constexpr int kKStages = 3, kVStages = 2;
+
+enum FwdBar {
+  B_QFULL0 = 0, B_QFULL1, B_QEMPTY0, B_QEMPTY1,
+  B_KFULL0, B_KFULL1, B_KFULL2, B_KEMPTY0, B_KEMPTY1, B_KEMPTY2,
+  B_VFULL0, B_VFULL1, B_VEMPTY0, B_VEMPTY1,
+  B_SFULL0, B_SFULL1,
+  B_PFULL0, B_PFULL1,                        // kv columns 0-63 of P(t) are in TMEM (group t & 1)
+  B_PREST0, B_PREST1,                        // kv columns 64-127 too
+  B_SEGDONE,                                 // every MMA of the segment has completed
+  B_XFULL,                                   // both groups' row maxima and sums of the segment are in shared memory
+  B_OFREE,                                   // both accumulators of the segment have been read
+  B_PART,                                    // this CTA's part of an item is in the workspace
+  B_LAST,                                    // ... and it is known whether it was the item's last part
+  B_COUNT
+};
+
+template <int D>
+struct SplitSmem {
+  static constexpr int kTileBytes = kTile * D * 2;     // one 128 x D tile
+  static constexpr int kBoxBytes = kTile * 64 * 2;     // one TMA box: 128 rows x 64 columns
+  static constexpr int kQ = 0;
+  static constexpr int kK = 2 * kTileBytes;
+  static constexpr int kV = kK + kKStages * kTileBytes;
+  static constexpr int kX = kV + kVStages * kTileBytes;       // float2 [group][row]: maximum, sum
+  static constexpr int kBars = kX + 2 * kTile * 8;
+  static constexpr int kTmemSlot = kBars + 8 * B_COUNT;
+  static constexpr int kAbort = kTmemSlot + 4;
+  static constexpr int kLast = kAbort + 4;
+  static constexpr int kStart = kLast + 4;                    // five ints: where this CTA's share starts
+  static constexpr int kTotal = kStart + 20;
+  static_assert(kTotal <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
+};
+
+// Walk over the segments of a CTA's share.  Items are ordered (batch row, head item, query tile, token block): items that
+// read the same K / V are neighbours.  Every role walks on its own.
+struct SegWalk {
+  int b, hd, qt, j;        // item: batch row, head (or group of packed heads), query tile, token block of the tile
+  int count, first, len;   // tiles of the item; the segment is tiles [first, first + len) of its list
+  int left;                // tiles of the share from this segment on
+  __device__ __forceinline__ bool more() const { return left > 0; }
+  __device__ __forceinline__ void init(const int* start, const FwdArgs& a, int share) {
+    b = start[0]; hd = start[1]; qt = start[2]; j = start[3]; first = start[4];
+    left = share;
+    count = __ldg(a.list.counts + (long long)b * a.list.n_outer_tiles + qt);
+    len = min(count - first, left);
+  }
+  __device__ __forceinline__ void next(const FwdArgs& a) {
+    left -= len;
+    if (left <= 0) return;
+    first = 0;
+    if (++j == a.token_blocks) {
+      j = 0;
+      const int n_outer = a.list.n_outer_tiles;
+      do {                                                // there are tiles left: a list with entries follows
+        if (++qt == n_outer) {
+          qt = 0;
+          if (++hd == a.head_items) {
+            hd = 0;
+            do { ++b; } while (__ldg(a.list.prefix + (long long)b * n_outer) == __ldg(a.list.prefix + (long long)(b + 1) * n_outer));
+          }
+        }
+        count = __ldg(a.list.counts + (long long)b * n_outer + qt);
+      } while (count == 0);
+    }
+    len = min(count, left);
+  }
+};
+
+// Mask bits of query token r for the 128 keys from c0 of a partial list entry without an element mask (the pool of masks was
+// used up: rare).  Not inlined, so that what it needs lives in no register of the tile loop.
+__device__ __noinline__ uint4 split_keep_slow(const FwdArgs* a, int b, int r, bool row_valid, int c0) {
+  const RowBounds rb = load_bounds(a->mask, b, min(r, a->tok.q_len - 1));
+  int q_seg = KVAX_B200_PADDING_SEGMENT_ID, q_pos = 0;
+  if (row_valid) {
+    q_seg = __ldg(a->tok.q_seg + (long long)b * a->tok.q_len + r);
+    q_pos = query_position(a->tok, b, r);
+  }
+  const int32_t* kv_seg = a->tok.kv_seg + (long long)b * a->tok.kv_len;
+  const int32_t* kv_pos = a->tok.sequential ? nullptr : a->tok.kv_pos + (long long)b * a->tok.kv_len;
+  uint32_t w[4];
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch)
+    w[ch] = keep_bits32<false>(rb, c0 + ch * 32, a->tok.kv_len, row_valid, q_seg, q_pos, kv_seg + c0 + ch * 32,
+                               kv_pos ? kv_pos + c0 + ch * 32 : nullptr);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <int D, bool kF16>
+__global__ void __launch_bounds__(kThreads, 1)
+attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                      const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FwdArgs a) {
+  using L = SplitSmem<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sQ = smem + L::kQ;
+  uint8_t* sK = smem + L::kK;
+  uint8_t* sV = smem + L::kV;
+  float2* xl = reinterpret_cast<float2*>(smem + L::kX);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kTmemSlot);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbort);
+  volatile int* s_last = reinterpret_cast<volatile int*>(smem + L::kLast);
+  int* s_start = reinterpret_cast<int*>(smem + L::kStart);
+
+  // The swizzled tiles need a 1024-byte aligned base and the layout leaves no slack to round up.
+  if (smem_u32(smem) & 1023u) {
+    if (threadIdx.x == 0) report_status(a.status, ST_SMEM_MISALIGNED);
+    return;
+  }
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_outer = a.list.n_outer_tiles;
+  const int n_rows = a.batch * n_outer;
+  const int row = tid & (kTile - 1);
+  const int wg = (tid >> 7) & 1;                         // softmax group; at the end of a segment also the column half
+  const int q_len = a.tok.q_len;
+
+  // Query tiles without any kv tile belong to no share: zeros (:253-258), the lists dealt out over the CTAs.
+  for (int lr = blockIdx.x; lr < n_rows; lr += gridDim.x) {
+    if (__ldg(a.list.counts + lr) != 0) continue;
+    const int zb = lr / n_outer, t0 = (lr % n_outer) * kTile;
+    const int n = min(kTile, q_len - t0) * a.q_heads;
+    for (int i = tid; i < n * (D / 8); i += kThreads) {
+      const int x = i / (D / 8), t = t0 + x / a.q_heads, h = x % a.q_heads;
+      __nv_bfloat16* o = a.out + (long long)zb * a.o_strides[0] + (long long)t * a.o_strides[1] + (long long)h * a.o_strides[2];
+      reinterpret_cast<uint4*>(o)[i % (D / 8)] = make_uint4(0, 0, 0, 0);
+      if (i % (D / 8) == 0) a.lse[((long long)zb * a.q_heads + h) * q_len + t] = a.empty_lse;
+    }
+  }
+
+  // This CTA's share of the sequence of tiles: [x0, x0 + share)
+  const int per_list = a.head_items * a.token_blocks;    // items per list
+  const int total = __ldg(a.list.prefix + n_rows) * per_list;
+  const int tiles_per_cta = max((total + int(gridDim.x) - 1) / int(gridDim.x), a.min_tiles);
+  const int x0 = int(blockIdx.x) * tiles_per_cta;
+  const int share = min(tiles_per_cta, total - x0);
+  if (share <= 0) return;
+  for (int i = tid; i < a.batch; i += kThreads) {
+    const int lo = __ldg(a.list.prefix + (long long)i * n_outer), hi = __ldg(a.list.prefix + (long long)(i + 1) * n_outer);
+    if (x0 >= lo * per_list && x0 < hi * per_list) s_start[0] = i;
+  }
+  if (tid == 0) {
+    for (int i = 0; i < B_COUNT; ++i) {
+      int n = 1;
+      if (i >= B_PFULL0 && i <= B_PREST1) n = kTile;
+      if (i == B_XFULL || i == B_OFREE || i == B_PART) n = kSoftmaxThreads;
+      mbar_init(&bars[i], n);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == kKWarp) tmem_alloc(tmem_slot, kTmemCols);
+  __syncthreads();
+  {
+    const int* pre = a.list.prefix + (long long)s_start[0] * n_outer;
+    const int p0 = __ldg(pre), w = (__ldg(pre + n_outer) - p0) * a.token_blocks;     // tiles per head of this batch row
+    const int rem = x0 - p0 * per_list, in_head = rem % w;
+    for (int i = tid; i < n_outer; i += kThreads) {
+      const int lo = (__ldg(pre + i) - p0) * a.token_blocks, n = __ldg(pre + i + 1) - __ldg(pre + i);
+      if (in_head >= lo && in_head < lo + n * a.token_blocks) {
+        s_start[1] = rem / w; s_start[2] = i; s_start[3] = (in_head - lo) / n; s_start[4] = (in_head - lo) % n;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;                 // scores of tile t of the share: tmem_base + 128 * (t & 1)
+  const uint32_t tO = tmem_base + 2 * kTile;             // accumulator of group g: tO + 128 * g
+
+  const int pack = a.pack, tile_tokens = a.tile_tokens;
+  SegWalk sw;
+  sw.init(s_start, a, share);
+  auto seg_list = [&]() {
+    return a.list.tiles + ((long long)sw.b * n_outer + sw.qt) * a.list.n_inner_tiles + sw.first;
+  };
+  // kv head of the segment's head item: `pack` heads of one group, or a single query head
+  auto seg_kv_head = [&]() { return sw.hd * pack / a.group; };
+
+  if (warp == kKWarp) {
+    // ------------------------------------------------------------------ Q and K producer
+    if (lane == 0) {
+      prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k);
+      const uint32_t q_bytes = uint32_t(tile_tokens * pack * 128 * (D / 64));
+      bool ok = true;
+      int t = 0;
+      for (int seg = 0; sw.more() && ok; ++seg, sw.next(a)) {
+        const int qb = seg & 1;
+        if (seg >= 2) ok = mbar_wait(&bars[B_QEMPTY0 + qb], ((seg >> 1) - 1) & 1, abort_flag, a.status, B_QEMPTY0 + qb);
+        if (!ok) break;
+        mbar_arrive_expect_tx(&bars[B_QFULL0 + qb], q_bytes);
+#pragma unroll
+        for (int x = 0; x < D / 64; ++x)
+          tma_load_4d(sQ + qb * L::kTileBytes + x * L::kBoxBytes, &tmap_q, &bars[B_QFULL0 + qb], x * 64, sw.hd * pack,
+                      sw.qt * kTile + sw.j * tile_tokens, sw.b);
+        const int kvh = seg_kv_head();
+        const uint32_t* list = seg_list();
+        uint32_t e_next = __ldg(list);               // list entries are fetched one iteration ahead
+        for (int i = 0; i < sw.len && ok; ++i, ++t) {
+          const int st = t % kKStages, use = t / kKStages;
+          const int u = int(e_next & a.list.tile_mask);
+          if (i + 1 < sw.len) e_next = ldg_pinned(list + i + 1);
+          if (use > 0) ok = mbar_wait(&bars[B_KEMPTY0 + st], (use - 1) & 1, abort_flag, a.status, B_KEMPTY0 + st);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&bars[B_KFULL0 + st], L::kTileBytes);
+#pragma unroll
+          for (int x = 0; x < D / 64; ++x)
+            tma_load_4d(sK + st * L::kTileBytes + x * L::kBoxBytes, &tmap_k, &bars[B_KFULL0 + st], x * 64, kvh, u * kTile, sw.b);
+        }
+      }
+    }
+  } else if (warp == kVWarp) {
+    // ------------------------------------------------------------------ V producer
+    if (lane == 0) {
+      prefetch_tmap(&tmap_v);
+      bool ok = true;
+      int t = 0;
+      for (; sw.more() && ok; sw.next(a)) {
+        const int kvh = seg_kv_head();
+        const uint32_t* list = seg_list();
+        uint32_t e_next = __ldg(list);
+        for (int i = 0; i < sw.len && ok; ++i, ++t) {
+          const int st = t % kVStages, use = t / kVStages;
+          const int u = int(e_next & a.list.tile_mask);
+          if (i + 1 < sw.len) e_next = ldg_pinned(list + i + 1);
+          if (use > 0) ok = mbar_wait(&bars[B_VEMPTY0 + st], (use - 1) & 1, abort_flag, a.status, B_VEMPTY0 + st);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&bars[B_VFULL0 + st], L::kTileBytes);
+#pragma unroll
+          for (int x = 0; x < D / 64; ++x)
+            tma_load_4d(sV + st * L::kTileBytes + x * L::kBoxBytes, &tmap_v, &bars[B_VFULL0 + st], x * 64, kvh, u * kTile, sw.b);
+        }
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    // ------------------------------------------------------------------ MMA issuer (whole warp; one elected lane issues)
+    constexpr uint32_t idesc_s = make_idesc_16(kTile, kTile, 0, 0, kF16);   // Q (K-major) x K (K-major)
+    constexpr uint32_t idesc_o = make_idesc_16(kTile, D, 0, 1, kF16);       // P (TMEM)    x V (N-major)
+    const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
+    bool ok = true;
+    auto wait = [&](int bar, uint32_t parity, bool tmem_sync) {
+      ok = mbar_wait(&bars[bar], parity, abort_flag, a.status, bar);
+      ok = __all_sync(0xffffffffu, ok);
+      if (tmem_sync) tc_fence_after();
+    };
+    // Scores run two tiles ahead of P V and cross into the next segment: a walk of their own.
+    SegWalk qw = sw;
+    int q_seg_no = 0, q_done = 0;                // segment of the next scores, tiles of it issued so far
+    auto issue_qk = [&](int t) {                 // scores of tile t of the share into buffer t & 1
+      const int qb = q_seg_no & 1;
+      if (q_done == 0) { wait(B_QFULL0 + qb, (q_seg_no >> 1) & 1, false); if (!ok) return; }
+      const int st = t % kKStages, use = t / kKStages;
+      wait(B_KFULL0 + st, use & 1, false);
+      if (!ok) return;
+      const bool seg_end = ++q_done == qw.len;
+      const uint32_t ts = tmem_base + (t & 1) * kTile;
+      const uint32_t q_lo = sdesc_lo_sw128(q_addr + qb * L::kTileBytes, 16);
+      const uint32_t k_lo = sdesc_lo_sw128(k_addr + st * L::kTileBytes, 16);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint32_t off = ((kk >> 2) * L::kBoxBytes + (kk & 3) * 32) >> 4;   // 16 elements = 32 B inside a 128 B row
+          umma_ss_lo(ts, q_lo + off, k_lo + off, idesc_s, kk > 0);
+        }
+        umma_commit(&bars[B_SFULL0 + (t & 1)]);
+        umma_commit(&bars[B_KEMPTY0 + st]);               // the K producer may refill the stage
+        if (seg_end) umma_commit(&bars[B_QEMPTY0 + qb]);  // ... and the Q buffer
+      }
+      __syncwarp();
+      if (seg_end) { qw.next(a); ++q_seg_no; q_done = 0; }
+    };
+    issue_qk(0);
+    if (ok && share > 1) issue_qk(1);
+    int t = 0;
+    for (int seg = 0; sw.more() && ok; ++seg, sw.next(a)) {
+      if (seg > 0) wait(B_OFREE, (seg - 1) & 1, true);    // the accumulators of the segment before have been read
+      if (!ok) break;
+      uint32_t acc[2] = {0u, 0u};
+      for (int i = 0; i < sw.len && ok; ++i, ++t) {
+        const int g = t & 1, vs = t % kVStages, vuse = t / kVStages;
+        wait(B_VFULL0 + vs, vuse & 1, false);
+        if (!ok) break;
+        wait(B_PFULL0 + g, (t >> 1) & 1, true);
+        if (!ok) break;
+        const uint32_t tp = tmem_base + g * kTile;
+        const uint32_t on = g ? acc[1] : acc[0];
+        // 16 kv rows per step: rows are 128 B apart, d columns 0-63 / 64-127 in separate boxes
+        const uint32_t v_lo = sdesc_lo_sw128(v_addr + vs * L::kTileBytes, L::kBoxBytes);
+        // P arrives in two halves: the first four k-steps run while the group still exponentiates the second half
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < kTile / 32; ++kk)
+            umma_ts_lo(tO + g * kTile, tp + kk * 8, v_lo + ((kk * 16 * 128) >> 4), idesc_o, (kk > 0) ? 1u : on);
+        }
+        __syncwarp();
+        wait(B_PREST0 + g, (t >> 1) & 1, true);
+        if (!ok) break;
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = kTile / 32; kk < kTile / 16; ++kk)
+            umma_ts_lo(tO + g * kTile, tp + kk * 8, v_lo + ((kk * 16 * 128) >> 4), idesc_o, 1u);
+          umma_commit(&bars[B_VEMPTY0 + vs]);
+          if (i + 1 == sw.len) umma_commit(&bars[B_SEGDONE]);
+        }
+        __syncwarp();
+        if (g) acc[1] = 1u; else acc[0] = 1u;
+        if (t + 2 < share) issue_qk(t + 2);      // reuses buffer g: issued after P V of tile t, which read P
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax groups, end of a segment
+    const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
+    const uint32_t tS = tmem_base + wg * kTile + lane_base;
+    const uint32_t tOg = tO + wg * kTile + lane_base;
+    const float c = a.scale_log2e;
+    const int row_token = row / pack, row_head = row - row_token * pack;
+    bool ok = true;
+    int t0 = 0, n_parts = 0;                     // tiles of the share before this segment; partial segments so far
+    for (int seg = 0; sw.more() && ok; ++seg, t0 += sw.len, sw.next(a)) {
+      // row of this thread: query token r of the batch row, query head h
+      const int tile_token = sw.j * tile_tokens + row_token;          // within the 128 tokens of the list's query tile
+      const int r = sw.qt * kTile + tile_token;
+      const int h = sw.hd * pack + row_head;
+      const bool row_valid = row_token < tile_tokens && r < q_len;
+      const bool live = __any_sync(0xffffffffu, row_valid);
+      const uint32_t* list = seg_list();
+
+      // Online softmax state of this group (see attn_fwd_one.cu): the reference maximum follows the true one lazily.
+      constexpr float kLazy = 8.f;
+      float m = -INFINITY, l = 0.f;
+      const int i0 = (t0 ^ wg) & 1;              // first tile of the segment that is this group's
+      uint32_t e_next = (i0 < sw.len) ? __ldg(list + i0) : 0u;
+      for (int i = i0; i < sw.len && ok; i += 2) {
+        const int t = t0 + i;
+        const uint32_t e = e_next;
+        if (i + 2 < sw.len) e_next = ldg_pinned(list + i + 2);
+        const int c0 = int(e & a.list.tile_mask) * kTile;
+        const bool partial = (e & kPartialBit) != 0;
+        uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+        if (partial && live) {
+          const uint4 w = (e & kBitmapBit) ? __ldg(entry_bitmap(a.list, e) + (tile_token & (kTile - 1)))
+                                           : split_keep_slow(&a, sw.b, r, row_valid, c0);
+          keep[0] = w.x; keep[1] = w.y; keep[2] = w.z; keep[3] = w.w;
+        }
+        ok = mbar_wait(&bars[B_SFULL0 + wg], (t >> 1) & 1, abort_flag, a.status, B_SFULL0 + wg);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        if (live) {
+          uint32_t v[4][32];
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) tmem_ld32(tS + ch * 32, v[ch]);
+          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            tmem_ld_wait(v[ch]);
+            if (partial) {
+#pragma unroll
+              for (int jj = 0; jj < 32; ++jj) v[ch][jj] = ((keep[ch] >> jj) & 1u) ? v[ch][jj] : 0xff800000u;   // -inf
+            }
+#pragma unroll
+            for (int jj = 0; jj < 32; jj += 8) {
+#pragma unroll
+              for (int x = 0; x < 4; ++x)
+                mx4[x] = fmax3(mx4[x], __uint_as_float(v[ch][jj + 2 * x]), __uint_as_float(v[ch][jj + 2 * x + 1]));
+            }
+          }
+          float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+          mx *= c;                                  // scale > 0
+          float alpha = 1.f;
+          if (mx - m > kLazy) {                     // also taken when m is still -inf
+            alpha = fast_exp2(m - mx);              // 0 when m was -inf
+            m = mx;
+          }
+          // The group's previous P V, of tile t - 2, was issued before the scores of tile t, which are here (a commit
+          // covers everything issued before it): it has completed and the accumulator may be rescaled.
+          if (i > i0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+            for (int ch = 0; ch < D / 16; ++ch) {
+              uint32_t o[16];
+              tmem_ld16(tOg + ch * 16, o);
+              tmem_ld_wait16(o);
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj) o[jj] = __float_as_uint(__uint_as_float(o[jj]) * alpha);
+              tmem_st16(tOg + ch * 16, o);
+            }
+          }
+          const float neg_m = (m == -INFINITY) ? 0.f : -m;
+          float rs4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int jj = 0; jj < 32; jj += 2) {
+              const float p0 = fast_exp2(fmaf(__uint_as_float(v[ch][jj]), c, neg_m));       // exp2(-inf) = 0 on masked columns
+              const float p1 = fast_exp2(fmaf(__uint_as_float(v[ch][jj + 1]), c, neg_m));
+              rs4[(jj >> 1) & 3] += p0 + p1;
+              pk[jj >> 1] = pack16<kF16>(p0, p1);
+            }
+            if (ch == 2) {                          // the first half of P (and the rescaled accumulator) is in TMEM by now
+              tmem_st_wait();
+              tc_fence_before();
+              mbar_arrive(&bars[B_PFULL0 + wg]);
+            }
+            tmem_st16(tS + ch * 16, pk);
+          }
+          l = l * alpha + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
+          tmem_st_wait();
+          tc_fence_before();
+          mbar_arrive(&bars[B_PREST0 + wg]);
+        } else {
+          tc_fence_before();
+          mbar_arrive(&bars[B_PFULL0 + wg]);
+          mbar_arrive(&bars[B_PREST0 + wg]);
+        }
+      }
+      if (!ok) break;
+
+      // ---- end of the segment: merge the two groups; every thread handles D/2 columns of its row
+      ok = mbar_wait(&bars[B_SEGDONE], seg & 1, abort_flag, a.status, B_SEGDONE);
+      if (ok) {
+        xl[wg * kTile + row] = make_float2(m, l);
+        mbar_arrive(&bars[B_XFULL]);
+        ok = mbar_wait(&bars[B_XFULL], seg & 1, abort_flag, a.status, B_XFULL);
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const float2 other = xl[(wg ^ 1) * kTile + row];
+      const float m0 = wg ? other.x : m, l0 = wg ? other.y : l;     // group 0 / group 1 state
+      const float m1 = wg ? m : other.x, l1 = wg ? l : other.y;
+      const float mt = fmaxf(m0, m1);
+      const float a0 = (l0 > 0.f) ? fast_exp2(m0 - mt) : 0.f;       // a group that saw nothing contributes nothing
+      const float a1 = (l1 > 0.f) ? fast_exp2(m1 - mt) : 0.f;
+      const float lt = l0 * a0 + l1 * a1;
+      const bool whole = sw.len == sw.count;                        // the item is this CTA's alone
+      const float inv = whole ? ((lt > 0.f) ? (1.f / lt) : 0.f) : 1.f;
+      const float w0 = a0 * inv, w1 = a1 * inv;
+      const uint32_t col0 = wg * (D / 2);
+      __nv_bfloat16* o_row = a.out + (long long)sw.b * a.o_strides[0] + (long long)r * a.o_strides[1] +
+                             (long long)h * a.o_strides[2] + col0;
+      // parts of an item: the CTA it starts in keeps its part in slot 1, the others in slot 0 (a CTA holds at most one of each)
+      const int slot = 2 * int(blockIdx.x) + (sw.first == 0 ? 1 : 0);
+      float* part = a.parts + ((long long)slot * kTile + row) * D + col0;
+      if (live) {
+#pragma unroll
+        for (int ch = 0; ch < D / 64; ++ch) {
+          uint32_t v0[32], v1[32];
+          tmem_ld32(tO + lane_base + col0 + ch * 32, v0);
+          tmem_ld32(tO + kTile + lane_base + col0 + ch * 32, v1);
+          tmem_ld_wait(v0);
+          tmem_ld_wait(v1);
+          if (row_valid) {
+            float o[32];
+#pragma unroll
+            for (int jj = 0; jj < 32; ++jj) {
+              const float y0 = (w0 != 0.f) ? __uint_as_float(v0[jj]) * w0 : 0.f;   // an unused accumulator holds garbage
+              const float y1 = (w1 != 0.f) ? __uint_as_float(v1[jj]) * w1 : 0.f;
+              o[jj] = y0 + y1;
+            }
+            if (whole) {
+#pragma unroll
+              for (int jj = 0; jj < 32; jj += 8) {
+                uint4 w;
+                w.x = pack16<kF16>(o[jj + 0], o[jj + 1]);
+                w.y = pack16<kF16>(o[jj + 2], o[jj + 3]);
+                w.z = pack16<kF16>(o[jj + 4], o[jj + 5]);
+                w.w = pack16<kF16>(o[jj + 6], o[jj + 7]);
+                reinterpret_cast<uint4*>(o_row)[(ch * 32 + jj) >> 3] = w;
+              }
+            } else {
+#pragma unroll
+              for (int jj = 0; jj < 32; jj += 4)
+                reinterpret_cast<float4*>(part)[(ch * 32 + jj) >> 2] = make_float4(o[jj], o[jj + 1], o[jj + 2], o[jj + 3]);
+            }
+          }
+        }
+        // A row that saw no unmasked key keeps O = 0 and gets LSE2 = +inf, so that the backward pass computes
+        // exp2(s - LSE2) = 0 for it.
+        if (row_valid && wg == 0) {
+          if (whole) a.lse[((long long)sw.b * a.q_heads + h) * q_len + r] = (lt > 0.f) ? (mt + __log2f(lt)) : INFINITY;
+          else a.part_ml[(long long)slot * kTile + row] = make_float2(mt, lt);
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(&bars[B_OFREE]);               // the next segment's P V may overwrite the accumulators
+      if (whole) continue;
+
+      // ---- part of an item: the CTA that finishes the last part merges all of them
+      const uint32_t part_phase = uint32_t(n_parts++ & 1);
+      const int item_x0 = x0 + t0 - sw.first;                       // where the item starts in the sequence of tiles
+      const int cta0 = item_x0 / tiles_per_cta, cta1 = (item_x0 + sw.count - 1) / tiles_per_cta;
+      __threadfence();
+      mbar_arrive(&bars[B_PART]);
+      ok = mbar_wait(&bars[B_PART], part_phase, abort_flag, a.status, B_PART);
+      if (ok && tid == 0) {
+        __threadfence();
+        *s_last = atomicAdd(a.part_counters + cta0, 1) == cta1 - cta0;
+        mbar_arrive(&bars[B_LAST]);
+      }
+      if (ok) ok = mbar_wait(&bars[B_LAST], part_phase, abort_flag, a.status, B_LAST);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok || !*s_last) continue;
+      __threadfence();
+      const int rows_used = min(tile_tokens, q_len - (sw.qt * kTile + sw.j * tile_tokens)) * pack;
+      constexpr int kVec = D / 4;
+      for (int x = tid; x < rows_used * kVec; x += kSoftmaxThreads) {
+        const int pr = x / kVec, vec = x % kVec;
+        auto part_row = [&](int p) { return (long long)(2 * p + (p == cta0 ? 1 : 0)) * kTile + pr; };
+        // maximum first, so that the parts are independent loads
+        float M = -INFINITY, Ls = 0.f;
+#pragma unroll 4
+        for (int p = cta0; p <= cta1; ++p) M = fmaxf(M, __ldcg(a.part_ml + part_row(p)).x);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int p = cta0; p <= cta1; ++p) {
+          const float2 ml = __ldcg(a.part_ml + part_row(p));
+          const float4 y = __ldcg(reinterpret_cast<const float4*>(a.parts + part_row(p) * D) + vec);
+          const float w = (ml.y > 0.f) ? fast_exp2(ml.x - M) : 0.f;   // a part that saw no unmasked key of the row holds zeros
+          acc.x += y.x * w; acc.y += y.y * w; acc.z += y.z * w; acc.w += y.w * w;
+          Ls += ml.y * w;
+        }
+        const float iv = (Ls > 0.f) ? (1.f / Ls) : 0.f;
+        const int tok = sw.qt * kTile + sw.j * tile_tokens + pr / pack, hq = sw.hd * pack + pr % pack;
+        __nv_bfloat16* o = a.out + (long long)sw.b * a.o_strides[0] + (long long)tok * a.o_strides[1] +
+                           (long long)hq * a.o_strides[2] + vec * 4;
+        *reinterpret_cast<uint2*>(o) = make_uint2(pack16<kF16>(acc.x * iv, acc.y * iv), pack16<kF16>(acc.z * iv, acc.w * iv));
+        if (vec == 0) a.lse[((long long)sw.b * a.q_heads + hq) * q_len + tok] = (Ls > 0.f) ? (M + __log2f(Ls)) : INFINITY;
+      }
+    }
+  }
+
+  // ---------------------------------------------------------------------- teardown
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kKWarp) {
+    // After an aborted run a TMA copy may still be in flight: give it a bounded moment
+    // before the CTA (and its shared memory) goes away.
+    if (*abort_flag && lane == 0) {
+      const uint64_t tw = globaltimer_ns();
+      while (globaltimer_ns() - tw < 200000ull) { }
+    }
+    __syncwarp();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+template <int D, bool kF16>
+int launch_split(const FwdLaunch& L, cudaStream_t stream) {
+  constexpr int smem = SplitSmem<D>::kTotal;
+  auto kern = attn_fwd_split_kernel<D, kF16>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return KVAX_B200_ELAUNCH;
+  kern<<<kSplitCtas, kThreads, smem, stream>>>(L.tmap_q, L.tmap_k, L.tmap_v, L.args);
+  return cudaGetLastError() == cudaSuccess ? KVAX_B200_OK : KVAX_B200_ELAUNCH;
+}
+
+}  // namespace
+
+int launch_attn_fwd_split(const FwdLaunch& L, cudaStream_t stream) {
+  const bool f16 = L.dtype == KVAX_B200_F16;
+  if (L.head_dim == 128) return f16 ? launch_split<128, true>(L, stream) : launch_split<128, false>(L, stream);
+  if (L.head_dim == 64) return f16 ? launch_split<64, true>(L, stream) : launch_split<64, false>(L, stream);
+  return KVAX_B200_EUNSUPPORTED;
+}
+
+}  // namespace kvx

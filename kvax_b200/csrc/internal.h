@@ -9,7 +9,9 @@
 
 namespace kvx {
 
-constexpr int kListCounters = 4;   // two per list of a call (the backward builds up to two)
+constexpr int kSplitCtas = 148;    // forward with the work split over the SMs: one CTA per SM,
+constexpr int kSplitMinTiles = 4;  // none with a smaller share than this (start-up would outweigh it)
+constexpr int kListCounters = 4 + kSplitCtas;   // two per list of a call (the backward builds up to two), one per CTA of the split forward
 
 struct ScheduleArgs {
   MaskView mask;
@@ -18,6 +20,7 @@ struct ScheduleArgs {
   int32_t* counts;     // (B, n_outer_tiles)
   int32_t* order;      // (B * n_outer_tiles) launch order of the rows (blocks of neighbours, longest lists first)
   int32_t* pair_order; // (B * ceil(n_outer_tiles / 2)) the same order for pairs (2p, 2p+1): row of the even tile
+  int32_t* prefix;     // written instead of the launch orders when not null: see TileList
   const int4* inner_summary;  // (B, n_inner_tiles) {seg_min, seg_max, pos_min, pos_max}
   int32_t* counters;   // [0] masks taken from the pool, [1] finished lists; zero on entry (launch_tile_summaries)
   uint4* bitmaps;      // (n_bitmaps, 128) pool of element masks, or null
@@ -40,6 +43,14 @@ struct FwdArgs {
   int32_t q_heads, group;   // group = Hq / Hkv
   int32_t batch;
   float empty_lse;          // log-sum-exp written for the rows of query tiles without any key tile (0, or +inf on request)
+  // split forward (attn_fwd_split.cu): a query tile is `tile_tokens` tokens x `pack` heads of a kv group (or 128 tokens of one head)
+  int32_t pack, tile_tokens;
+  int32_t token_blocks;     // such tiles per list
+  int32_t head_items;       // heads / pack
+  int32_t min_tiles;        // no CTA takes a smaller share than this
+  float* parts;             // (2 * kSplitCtas, 128, D) parts of items that several CTAs work on
+  float2* part_ml;          // (2 * kSplitCtas, 128) their row maxima and sums
+  int32_t* part_counters;   // (kSplitCtas) finished parts, zero on entry
   int32_t pair_heads;       // pair kernel: a CTA takes one query tile of two heads of a kv group instead of two tiles of one head
 };
 
@@ -51,6 +62,8 @@ struct FwdLaunch {
 // CTAs of two neighbouring query tiles that share their K / V tiles (attn_fwd.cu), or of one query tile (attn_fwd_one.cu).
 int launch_attn_fwd(const FwdLaunch& L, cudaStream_t stream);
 int launch_attn_fwd_one(const FwdLaunch& L, cudaStream_t stream);
+// The kv tiles of all query tiles divided evenly over one CTA per SM (attn_fwd_split.cu).
+int launch_attn_fwd_split(const FwdLaunch& L, cudaStream_t stream);
 
 struct BwdArgs {
   TileList list;            // dQ kernel: one row per query tile; dK/dV kernel: per kv tile

@@ -80,15 +80,16 @@ def get_context_parallel_overlap() -> bool:
     return _cp_overlap
 
 
-_FWD_KERNELS = ("auto", "one_tile", "tile_pairs", "head_pairs")
+_FWD_KERNELS = ("auto", "one_tile", "tile_pairs", "head_pairs", "split")
 _fwd_kernel = "auto"
 
 
 def set_forward_kernel(kernel: str) -> None:
     """Which forward kernel runs: a CTA per 128-row query tile ("one_tile"); a CTA per two work items that share
     their K / V tiles -- two neighbouring query tiles of one head ("tile_pairs") or one query tile of two query heads
-    of a kv group ("head_pairs", grouped-query attention with an even group); or the library's choice ("auto",
-    default: head pairs when the group is even and at least two CTAs per SM remain, else pairs from 16k kv tokens
+    of a kv group ("head_pairs", grouped-query attention with an even group); the kv tiles of all query tiles divided
+    evenly over one CTA per SM ("split", for few query tiles on many keys); or the library's choice ("auto",
+    default: split for few queries on long keys -- decoding, small chunks of a prompt --, else head pairs when the group is even and at least two CTAs per SM remain, else pairs from 16k kv tokens
     on, else one tile).  Same results to rounding either way."""
     global _fwd_kernel
     if kernel not in _FWD_KERNELS:
@@ -314,7 +315,7 @@ def attention_forward(q, k, v, q_pos, q_seg, kv_pos, kv_seg, mask_fwd: Attention
     p = _lib.AttnFwdParams()
     p.stages = int(stages)
     p.flags = {"auto": 0, "one_tile": _lib.FWD_ONE_TILE, "tile_pairs": _lib.FWD_TILE_PAIRS,
-               "head_pairs": _lib.FWD_HEAD_PAIRS}[kernel or _fwd_kernel] | (_lib.FWD_EMPTY_LSE_INF if empty_lse_inf else 0)
+               "head_pairs": _lib.FWD_HEAD_PAIRS, "split": _lib.FWD_SPLIT}[kernel or _fwd_kernel] | (_lib.FWD_EMPTY_LSE_INF if empty_lse_inf else 0)
     _fill_shape(p.shape, q, k, v, out, q_pos, q_seg, kv_pos, kv_seg, scale, assume_sequential_positions, offsets)
     p.q, p.k, p.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
     p.mask, keep = _block_mask(mask_fwd, *fwd_blocks)

@@ -1,0 +1,82 @@
+"""The forward kernel that divides the kv tiles of all query tiles evenly over the SMs, where it can go wrong: heads of a
+group packed into one tile (groups that do and do not divide it, token counts around its edges), one item over many CTAs,
+many items in one CTA, rows without keys."""
+import pytest
+import torch
+
+from helpers import compare
+from oracle import attention_oracle as ao
+
+pytestmark = pytest.mark.gpu
+
+# batch, q_len, kv_len, q_heads, kv_heads, head_dim, dtype
+CASES = [
+    (3, 1, 1090, 8, 2, 128, torch.bfloat16),        # decoding; one row of a group's four heads
+    (2, 7, 200, 6, 2, 64, torch.float16),           # three heads: 32 tokens x 3 = 96 rows of a tile
+    (2, 32, 700, 8, 2, 128, torch.bfloat16),        # a packed tile exactly full
+    (2, 33, 700, 8, 2, 128, torch.float16),         # ... and one token more: two token blocks
+    (1, 128, 900, 16, 2, 128, torch.bfloat16),      # eight token blocks: as many tiles as heads, not packed
+    (2, 200, 1090, 4, 2, 64, torch.bfloat16),       # two query tiles, the last one cut
+    (1, 1, 40000, 4, 1, 128, torch.bfloat16),       # one item over up to 79 CTAs
+    (1, 300, 20011, 2, 1, 128, torch.float16),      # items over several CTAs each
+    (9, 150, 190, 16, 16, 64, torch.bfloat16),      # more items than CTAs, several items each
+]
+
+
+def _tokens(batch, q_len, kv_len, seed):
+    """Keys: two or three documents and padding; queries: the last tokens before the padding."""
+    g = torch.Generator().manual_seed(seed)
+    pos = torch.arange(kv_len, dtype=torch.int32).repeat(batch, 1)
+    seg = torch.full((batch, kv_len), -1, dtype=torch.int32)
+    q_pos, q_seg = torch.zeros((batch, q_len), dtype=torch.int32), torch.zeros((batch, q_len), dtype=torch.int32)
+    for b in range(batch):
+        used = int(torch.randint(max(q_len, kv_len * 3 // 4), kv_len + 1, (1,), generator=g))
+        cut = int(torch.randint(0, used // 3 + 1, (1,), generator=g))
+        seg[b, :used] = 1
+        seg[b, :cut] = 0
+        q_pos[b], q_seg[b] = pos[b, used - q_len:used], seg[b, used - q_len:used]
+    return q_pos.cuda(), q_seg.cuda(), pos.cuda(), seg.cuda()
+
+
+def _run(case, tokens, kernel, seed, **kw):
+    from kvax_b200.ops.flash_attention import attention_forward, check_status
+    from kvax_b200.ops.mask_creator import build_masks
+
+    batch, q_len, kv_len, hq, hkv, d, dtype = case
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(batch, n, h, d, generator=g, device="cuda").to(dtype) for n, h in ((q_len, hq), (kv_len, hkv), (kv_len, hkv)))
+    masks = build_masks(*tokens, [(128, 128, False)], True)
+    out, lse, status = attention_forward(q, k, v, *tokens, masks[0], (128, 128), d ** -0.5, kernel=kernel, **kw)
+    torch.cuda.synchronize()
+    check_status(status, "attention")
+    return q, k, v, out, lse
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_split(case):
+    tokens = _tokens(*case[:3], seed=sum(case[:3]))
+    q, k, v, out, lse = _run(case, tokens, "split", 5)
+    ref = ao.attention_dense_torch(q.float(), k.float(), v.float(), *tokens, case[5] ** -0.5)
+    compare("out", out.float().cpu().numpy(), ref["out"].cpu().numpy(), bf16_output=True)
+    # same scores, fp32 sums of up to 40000 terms in another order: 2^-24 * sqrt(40000) relative, log2 of it, scores of about 2^4
+    torch.testing.assert_close(lse, ref["lse2"], rtol=0, atol=1e-4)
+
+
+@pytest.mark.parametrize("empty_lse_inf", [False, True])
+def test_split_rows_without_keys(empty_lse_inf):
+    case = (3, 5, 1500, 8, 2, 128, torch.bfloat16)
+    tokens = _tokens(*case[:3], seed=3)
+    tokens[3][1] = -1                                # no key of the second row belongs to a document
+    got = _run(case, tokens, "split", 6, empty_lse_inf=empty_lse_inf)
+    want = _run(case, tokens, "one_tile", 6, empty_lse_inf=empty_lse_inf)
+    assert torch.equal(got[3][1], want[3][1]) and torch.equal(got[4][1], want[4][1])
+    assert not got[3][1].any()
+    compare("out", got[3].float().cpu().numpy(), want[3].float().cpu().numpy(), bf16_output=True)
+
+
+def test_split_is_the_default_for_few_queries():
+    """What `auto` takes and the forced kernel give the same bits where nothing is merged in a varying order."""
+    case = (2, 1, 3000, 8, 2, 128, torch.bfloat16)
+    tokens = _tokens(*case[:3], seed=4)
+    auto, split = _run(case, tokens, None, 7), _run(case, tokens, "split", 7)
+    assert torch.equal(auto[3], split[3]) and torch.equal(auto[4], split[4])
