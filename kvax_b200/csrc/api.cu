@@ -423,6 +423,11 @@ extern "C" int kvax_b200_attn_bwd(const kvax_b200_attn_bwd_params* p, void* work
       F.tmap_k = tk; F.tmap_v = tv; F.tmap_q = tq; F.tmap_do = tdo;
       rc = make_tmap_acc(&F.tmap_dq, dq_acc, s.batch, s.q_len, s.q_heads, s.head_dim);
       if (rc) return rc;
+      F.tmap_dk = F.tmap_dv = F.tmap_dq;
+      if (dk_acc) {
+        rc = make_tmap_acc(&F.tmap_dk, dk_acc, s.batch, s.kv_len, s.kv_heads, s.head_dim); if (rc) return rc;
+        rc = make_tmap_acc(&F.tmap_dv, dv_acc, s.batch, s.kv_len, s.kv_heads, s.head_dim); if (rc) return rc;
+      }
       F.batch = s.batch; F.head_dim = s.head_dim; F.dtype = s.dtype;
       rc = launch_attn_bwd_fused(F, st);
       if (rc) return rc;

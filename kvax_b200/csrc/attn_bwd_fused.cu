@@ -32,6 +32,15 @@
 // S^T(i+1) -> P^T(i+1) -> dV(i+1) overlaps.
 // Shared memory (D = 128): K, V 64 KB + 2 x Q 64 KB + dO 32 KB + dS^T 32 KB + drain staging 32 KB +
 // LSE2 / delta 2 KB.
+// What bounds it at D = 128 (4500 clk per item on the 32k document-mask workload, 2560 of them MMA): Q(i+1) arrives
+// late, because its stage is only free after dK(i-1) and a tile takes ~2500 clk to come from L2; taking dK before dQ moves
+// that wait to the drain and gains nothing, and the reduce-adds themselves take 3200 clk, close to the rate at which L2 adds
+// fp32 (3.5 KB per clock over the GPU, measured alone: 2800 clk per item).
+//
+// head_dim 64: the same kernel with the room that is left over: three Q stages, two dO stages, two dS^T tiles, and TMEM
+// T1 | T2 | dV | dK | dQ | dQ with dQ in columns of its own, so that dP^T(i+1) is issued as soon as dS^T(i) is written and
+// nothing waits for the drain but the dQ two items later.  8 x 2112 tokens, 16 heads, fp16, packed: 412 us as the dQ and dK/dV
+// kernel pair, 188 us.
 //
 // dQ is accumulated with fp32 atomics at L2, so its summation order (and last bits) vary from run
 // to run; dK and dV are accumulated in TMEM in a fixed order.
@@ -111,6 +120,8 @@ struct FusedSmem {
   static constexpr int kAbort = kTmemSlot + 4;
   static constexpr int kTotal = kAbort + 4;
   static_assert(kTotal <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
+  // the epilogue's boxes: two per register-math warp and 64 columns, in the buffers between K / V and the drain's staging
+  static_assert(kComputeWarps * (D / 64) * 2 * kStageBuf <= kStage - kQ, "dK / dV boxes do not fit the idle buffers");
 };
 
 // Mask bits of kv row r for the 64 queries [i0, i0 + 64) of a partial list entry that carries no element mask from the
@@ -133,7 +144,8 @@ template <int D, bool kF16>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                       const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ BwdArgs a) {
+                      const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ CUtensorMap tmap_dk,
+                      const __grid_constant__ CUtensorMap tmap_dv, const __grid_constant__ BwdArgs a) {
   using L = FusedSmem<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
@@ -544,13 +556,27 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         tmem_ld32(tDK + lane_base + half * (D / 2) + ch * 32, v2);
         tmem_ld_wait(v1);
         tmem_ld_wait(v2);
-        if (row_valid && a.dkdv_accumulate) {
+        if (a.dkdv_accumulate) {
+          // Parts of several CTAs meet in fp32 accumulators: the warp's 32 x 32 boxes go through shared memory (the Q, dO and dS^T
+          // buffers are idle by now) and are added by TMA.  (Reductions straight from registers, a row per lane, ran at half
+          // the rate: 5900 clk for 128 x 128 floats per SM, measured alone, against 2800 for whole 128-byte lines.)
+          uint8_t* box = smem + L::kQ + ((warp * (D / 64) + ch) * 2) * kStageBuf;
+          auto put = [&](uint8_t* dst, const uint32_t (&x)[32], float f) {
 #pragma unroll
-          for (int jj = 0; jj < 32; jj += 4) {
-            red_add_f32x4(dv_row + ch * 32 + jj, __uint_as_float(v1[jj]), __uint_as_float(v1[jj + 1]), __uint_as_float(v1[jj + 2]),
-                          __uint_as_float(v1[jj + 3]));
-            red_add_f32x4(dk_row + ch * 32 + jj, __uint_as_float(v2[jj]) * a.scale, __uint_as_float(v2[jj + 1]) * a.scale,
-                          __uint_as_float(v2[jj + 2]) * a.scale, __uint_as_float(v2[jj + 3]) * a.scale);
+            for (int ck = 0; ck < 8; ++ck)
+              *reinterpret_cast<float4*>(dst + lane * 128 + ((ck ^ (lane & 7)) << 4)) =
+                  make_float4(__uint_as_float(x[4 * ck]) * f, __uint_as_float(x[4 * ck + 1]) * f, __uint_as_float(x[4 * ck + 2]) * f,
+                              __uint_as_float(x[4 * ck + 3]) * f);
+          };
+          put(box, v1, 1.f);
+          put(box + kStageBuf, v2, a.scale);
+          fence_proxy_async_smem();
+          __syncwarp();
+          const int r0 = kt * kTile + (warp & 3) * 32, col = half * (D / 2) + ch * 32;
+          if (lane == 0 && r0 < a.tok.kv_len) {               // rows beyond the sequence are clipped by TMA
+            tma_reduce_add_4d(&tmap_dv, box, col, kvh, r0, b);
+            tma_reduce_add_4d(&tmap_dk, box + kStageBuf, col, kvh, r0, b);
+            bulk_commit_group();
           }
         } else if (row_valid) {
           if (a.dkdv_16bit) {
@@ -581,6 +607,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         }
       }
     }
+    if (a.dkdv_accumulate && lane == 0) bulk_wait_group<0>();  // performed before the CTA goes away
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ dQ drain (warps 8-11)
     const int dw = warp - kDrainWarp0;                        // = TMEM lane quarter of this warp
@@ -707,7 +735,7 @@ int launch_fused(const FusedBwdLaunch& L, cudaStream_t stream) {
   auto kern = attn_bwd_fused_kernel<D, kF16>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return KVAX_B200_ELAUNCH;
   dim3 grid(L.args.list.n_outer_tiles * L.batch * L.args.kv_heads * L.args.head_split, 1, 1);
-  kern<<<grid, kThreads, smem, stream>>>(L.tmap_k, L.tmap_v, L.tmap_q, L.tmap_do, L.tmap_dq, L.args);
+  kern<<<grid, kThreads, smem, stream>>>(L.tmap_k, L.tmap_v, L.tmap_q, L.tmap_do, L.tmap_dq, L.tmap_dk, L.tmap_dv, L.args);
   return cudaGetLastError() == cudaSuccess ? KVAX_B200_OK : KVAX_B200_ELAUNCH;
 }
 

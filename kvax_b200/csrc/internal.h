@@ -100,6 +100,7 @@ int launch_attn_bwd_delta(const __nv_bfloat16* o, const __nv_bfloat16* d_o, floa
 // fp32 dQ accumulator (B, Sq, Hq, D), boxes of 32 rows x 32 columns, 128-byte swizzle.
 struct FusedBwdLaunch {
   CUtensorMap tmap_k, tmap_v, tmap_q, tmap_do, tmap_dq;
+  CUtensorMap tmap_dk, tmap_dv;   // fp32 dK / dV accumulators (dkdv_accumulate; else unused)
   BwdArgs args;             // list / mask: the kv-outer ones
   int batch, head_dim, dtype;
 };
