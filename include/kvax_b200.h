@@ -144,6 +144,17 @@ int kvax_b200_regroup_heads(const void* src, void* dst, int64_t tokens, int32_t 
 int kvax_b200_attn_merge(void* out_a, float* lse_a, const void* out_b, const float* lse_b, int64_t batch, int64_t seq,
                          int32_t heads, int32_t head_dim, int32_t dtype, kvax_b200_stream_t stream);
 
+/* Conversions around the attention entry points for fp32 tensors (the reference hands those to tl.dot as they are,
+ * flash_attention_triton.py:292-364).  All tensors dense, all pointers device memory.
+ *   abs_max:          *amax = largest magnitude of up to three fp32 tensors (`sizes` in elements; NaN if there is one)
+ *   scale_to_operand: y = x * s rounded to the 16-bit `dtype`, s the power of two that brings *amax to [1, 2)
+ *                     (amax clamped to 1e-30 from below); *inv = 1 / s
+ *   widen_to_float:   y = x * *inv in fp32 (inv may be null: 1) */
+int kvax_b200_abs_max(const float* const* tensors, const int64_t* sizes, int32_t n_tensors, float* amax, kvax_b200_stream_t stream);
+int kvax_b200_scale_to_operand(const float* x, int64_t n, const float* amax, int32_t dtype, void* y, float* inv,
+                               kvax_b200_stream_t stream);
+int kvax_b200_widen_to_float(const void* x, int64_t n, int32_t dtype, const float* inv, float* y, kvax_b200_stream_t stream);
+
 /* Head exchange over peer memory (no counterpart in the reference; it moves the data the
  * reference's all-gather of K / V moves, flash_attention_triton.py:2064-2115, for the
  * head-exchange schedule): one kernel reads a tensor of this GPU and stores every token's heads

@@ -29,6 +29,9 @@ EXPORTS = (
     "kvax_b200_attn_fwd",
     "kvax_b200_attn_bwd_workspace_bytes",
     "kvax_b200_attn_bwd",
+    "kvax_b200_abs_max",
+    "kvax_b200_scale_to_operand",
+    "kvax_b200_widen_to_float",
     "kvax_b200_wait_probe",
     "kvax_b200_host_word_device_pointer",
 )
@@ -130,6 +133,12 @@ def load() -> C.CDLL:
     lib.kvax_b200_attn_bwd_workspace_bytes.argtypes = [C.POINTER(AttnBwdParams)]
     lib.kvax_b200_attn_bwd.restype = C.c_int
     lib.kvax_b200_attn_bwd.argtypes = [C.POINTER(AttnBwdParams), vp, C.c_size_t, vp]
+    lib.kvax_b200_abs_max.restype = C.c_int
+    lib.kvax_b200_abs_max.argtypes = [C.POINTER(vp), C.POINTER(i64), i32, vp, vp]
+    lib.kvax_b200_scale_to_operand.restype = C.c_int
+    lib.kvax_b200_scale_to_operand.argtypes = [vp, i64, vp, i32, vp, vp, vp]
+    lib.kvax_b200_widen_to_float.restype = C.c_int
+    lib.kvax_b200_widen_to_float.argtypes = [vp, i64, i32, vp, vp, vp]
     lib.kvax_b200_wait_probe.restype = C.c_int
     lib.kvax_b200_wait_probe.argtypes = [vp, vp, i64, i32, vp]
     lib.kvax_b200_host_word_device_pointer.restype = C.c_int

@@ -120,11 +120,25 @@ def get_fp32_operand_dtype() -> str:
     return _fp32_operands
 
 
+def _abs_max(*tensors) -> torch.Tensor:
+    """Largest magnitude of up to three tensors, as an fp32 tensor of one element (one launch)."""
+    device = tensors[0].device
+    if any(t.device != device for t in tensors):
+        raise _lib.KvaxB200Error("query, key and value must be on one device")
+    ts = [t.detach().to(torch.float32).contiguous() for t in tensors]
+    out = torch.empty(1, dtype=torch.float32, device=device)
+    ptrs = (_lib.vp * len(ts))(*(t.data_ptr() for t in ts))
+    sizes = (_lib.i64 * len(ts))(*(t.numel() for t in ts))
+    with torch.cuda.device(device):
+        rc = _lib.load().kvax_b200_abs_max(ptrs, sizes, len(ts), out.data_ptr(), torch.cuda.current_stream(device).cuda_stream)
+    _lib.check(rc, "kvax_b200_abs_max")
+    return out
+
+
 def _fp32_operand_dtype(q, k, v) -> torch.dtype:
     if _fp32_operands != "auto":
         return torch.float16 if _fp32_operands == "float16" else torch.bfloat16
-    amax = torch.stack([t.detach().abs().amax() for t in (q, k, v)]).max().item()
-    return torch.float16 if amax <= 16384.0 else torch.bfloat16
+    return torch.float16 if _abs_max(q, k, v).item() <= 16384.0 else torch.bfloat16
 
 
 class _GradScaleBox:
@@ -143,9 +157,18 @@ class _ToOperand(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        inv = ctx.box.inv
+        if ctx.in_dtype == torch.float32 and g.dtype in (torch.float16, torch.bfloat16) and g.is_contiguous() and g.numel():
+            out = torch.empty_like(g, dtype=torch.float32)
+            with torch.cuda.device(g.device):
+                rc = _lib.load().kvax_b200_widen_to_float(g.data_ptr(), g.numel(), _lib.DTYPE_F16 if g.dtype == torch.float16 else _lib.DTYPE_BF16,
+                                                          None if inv is None else inv.data_ptr(), out.data_ptr(),
+                                                          torch.cuda.current_stream(g.device).cuda_stream)
+            _lib.check(rc, "kvax_b200_widen_to_float")
+            return out, None, None
         g = g.to(ctx.in_dtype)
-        if ctx.box.inv is not None:
-            g = g * ctx.box.inv
+        if inv is not None:
+            g = g * inv
         return g, None, None
 
 
@@ -157,13 +180,19 @@ class _FromOperand(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        if ctx.op_dtype == torch.float16:
-            # largest magnitude -> [1, 2): small gradients keep their bits, nothing overflows; exact (power of two)
-            amax = g.abs().amax().clamp_min(1e-30)
-            s = torch.exp2(-torch.floor(torch.log2(amax)))
-            ctx.box.inv = 1.0 / s
-            g = g * s
-        return g.to(ctx.op_dtype), None, None
+        if ctx.op_dtype != torch.float16:
+            return g.to(ctx.op_dtype), None, None
+        # largest magnitude -> [1, 2): small gradients keep their bits, nothing overflows; exact (power of two)
+        g = g.contiguous()
+        amax = _abs_max(g)
+        out = torch.empty_like(g, dtype=torch.float16)
+        inv = torch.empty_like(amax)
+        with torch.cuda.device(g.device):
+            rc = _lib.load().kvax_b200_scale_to_operand(g.data_ptr(), g.numel(), amax.data_ptr(), _lib.DTYPE_F16, out.data_ptr(),
+                                                        inv.data_ptr(), torch.cuda.current_stream(g.device).cuda_stream)
+        _lib.check(rc, "kvax_b200_scale_to_operand")
+        ctx.box.inv = inv
+        return out, None, None
 
 
 _HX_TRANSPORTS = ("auto", "peer", "nccl")
