@@ -92,7 +92,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int row_rank, kvh;
-  decode_block(blockIdx.x, a.list.n_outer_tiles * a.batch, a.kv_heads, &row_rank, &kvh);
+  decode_block(blockIdx.x, a.list.row_chunk, a.list.n_outer_tiles * a.batch, a.kv_heads, &row_rank, &kvh);
   const long long list_row = __ldg(a.list.order + row_rank);     // longest lists first
   const int b = int(list_row / a.list.n_outer_tiles), kt = int(list_row % a.list.n_outer_tiles);
   const int group = a.group;
@@ -490,7 +490,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int row_rank, h;
-  decode_block(blockIdx.x, a.list.n_outer_tiles * a.batch, a.q_heads, &row_rank, &h);
+  decode_block(blockIdx.x, a.list.row_chunk, a.list.n_outer_tiles * a.batch, a.q_heads, &row_rank, &h);
   const long long list_row = __ldg(a.list.order + row_rank);     // longest lists first
   const int b = int(list_row / a.list.n_outer_tiles), qt = int(list_row % a.list.n_outer_tiles);
   const int kvh = h / a.group;

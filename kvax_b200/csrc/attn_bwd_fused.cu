@@ -163,7 +163,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   // With `head_split` > 1 the query heads of a kv head are divided over that many CTAs (short or few lists would
   // otherwise leave SMs idle behind a few long CTAs); their dK / dV parts meet in fp32 accumulators by atomic adds.
   int row_rank, hh;
-  decode_block(blockIdx.x, a.list.n_outer_tiles * a.batch, a.kv_heads * a.head_split, &row_rank, &hh);
+  decode_block(blockIdx.x, a.list.row_chunk, a.list.n_outer_tiles * a.batch, a.kv_heads * a.head_split, &row_rank, &hh);
   const int kvh = hh / a.head_split;
   const long long list_row = __ldg(a.list.order + row_rank);     // longest lists first
   const int b = int(list_row / a.list.n_outer_tiles), kt = int(list_row % a.list.n_outer_tiles);

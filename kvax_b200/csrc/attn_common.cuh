@@ -184,6 +184,7 @@ struct TileList {
   const uint4* bitmaps;        // (pool, 128) element masks of marked entries, or null: none marked
   uint32_t tile_mask;          // low `tile_bits` bits of an entry
   int32_t tile_bits;
+  int32_t row_chunk;           // outer tiles that are launched as one block of neighbours: even, at most kRowChunk
   int32_t n_outer_tiles, n_inner_tiles;
 };
 
@@ -193,19 +194,19 @@ __device__ __forceinline__ const uint4* entry_bitmap(const TileList& l, uint32_t
 }
 
 // Launch geometry shared by the attention kernels: a 1-D grid over (outer tile, head).
-// Outer tiles are taken in the launch order built by schedule.cu (blocks of kRowChunk
-// neighbouring tiles, the blocks with the longest lists first), in chunks of kRowChunk; inside
+// Outer tiles are taken in the launch order built by schedule.cu (blocks of `row_chunk`
+// neighbouring tiles, the blocks with the longest lists first), in chunks of as many; inside
 // a chunk the heads are the slow index.  CTAs resident at the same time therefore belong to a
 // few heads and neighbouring outer tiles, so they stream the same inner tiles (served by L2),
 // while long work items still start early in the launch.
 constexpr int kRowChunk = 32;
-__device__ __forceinline__ void decode_block(int linear, int n_rows, int n_heads, int* row_rank, int* head) {
-  const int per_chunk = kRowChunk * n_heads;
+__device__ __forceinline__ void decode_block(int linear, int row_chunk, int n_rows, int n_heads, int* row_rank, int* head) {
+  const int per_chunk = row_chunk * n_heads;
   const int chunk = linear / per_chunk;
   const int within = linear - chunk * per_chunk;
-  const int rows_here = min(kRowChunk, n_rows - chunk * kRowChunk);
+  const int rows_here = min(row_chunk, n_rows - chunk * row_chunk);
   *head = within / rows_here;
-  *row_rank = chunk * kRowChunk + (within - *head * rows_here);
+  *row_rank = chunk * row_chunk + (within - *head * rows_here);
 }
 
 }  // namespace kvx

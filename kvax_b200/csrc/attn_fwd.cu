@@ -150,7 +150,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   // the same tile list, every K / V tile serves both and no union entry is ever one-sided.
   const int ph = a.pair_heads ? 1 : 0;
   int pair_rank, hh;
-  decode_block(blockIdx.x, (ph ? n_outer : (n_outer + 1) / 2) * a.batch, ph ? a.q_heads / 2 : a.q_heads, &pair_rank, &hh);
+  decode_block(blockIdx.x, a.list.row_chunk, (ph ? n_outer : (n_outer + 1) / 2) * a.batch, ph ? a.q_heads / 2 : a.q_heads, &pair_rank, &hh);
   const long long row0 = __ldg((ph ? a.list.order : a.list.pair_order) + pair_rank);     // list row of item 0
   const int b = int(row0 / n_outer), qt0 = int(row0 % n_outer);
   const bool has1 = ph || qt0 + 1 < n_outer;

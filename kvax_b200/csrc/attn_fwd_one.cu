@@ -82,7 +82,7 @@ attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int row_rank, h;
-  decode_block(blockIdx.x, a.list.n_outer_tiles * a.batch, a.q_heads, &row_rank, &h);
+  decode_block(blockIdx.x, a.list.row_chunk, a.list.n_outer_tiles * a.batch, a.q_heads, &row_rank, &h);
   const long long list_row = __ldg(a.list.order + row_rank);       // longest lists first
   const int b = int(list_row / a.list.n_outer_tiles), qt = int(list_row % a.list.n_outer_tiles);
   const int kvh = h / a.group;

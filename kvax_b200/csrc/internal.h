@@ -25,6 +25,7 @@ struct ScheduleArgs {
   int32_t* counters;   // [0] masks taken from the pool, [1] finished lists; zero on entry (launch_tile_summaries)
   uint4* bitmaps;      // (n_bitmaps, 128) pool of element masks, or null
   int32_t n_bitmaps, tile_bits;
+  int32_t row_chunk;   // see TileList: even, at most kRowChunk
   int32_t n_outer_tiles, n_inner_tiles;
   int32_t outer_len, inner_len;
 };

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) tile_summary_kernel(const TokenInfo tok, 
   if (lane == 0) (is_q ? q_sum : kv_sum)[local] = make_int4(smin, smax, pmin, pmax);
 }
 
-// Launch order.  Outer tiles are launched in blocks of kRowChunk neighbours (same batch row, consecutive tile
+// Launch order.  Outer tiles are launched in blocks of `row_chunk` neighbours (same batch row, consecutive tile
 // indices), the blocks sorted by their mean list length, longest first: the tail of a launch is then made of short
 // work items, and the CTAs that are resident together belong to neighbouring outer tiles of a few heads, which walk
 // through the same inner tiles (one document) -- their loads hit in L2 and, in the fused backward, their reduce-adds
@@ -79,15 +79,15 @@ struct OrderSmem {
   int warp_tot[kWarps], warp_tot2[kWarps];
 };
 
-__device__ void launch_order(OrderSmem& sm, const int32_t* counts, int32_t* order, int32_t* pair_order, int n_outer, int batch) {
+__device__ void launch_order(OrderSmem& sm, const int32_t* counts, int32_t* order, int32_t* pair_order, int n_outer, int batch, int row_chunk) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int blocks_per_row = (n_outer + kRowChunk - 1) / kRowChunk;
+  const int blocks_per_row = (n_outer + row_chunk - 1) / row_chunk;
   const int n_blocks = blocks_per_row * batch;
-  static_assert(kRowChunk == 32, "one lane per row of a block");
+  static_assert(kRowChunk <= 32, "one lane per row of a block");
   // whole warp; returns the key (mean list length, clamped).  The counts come from other CTAs: read past L1.
   auto block_info = [&](int blk, int* first_row, int* rows) -> int {
-    const int b = blk / blocks_per_row, t0 = (blk - b * blocks_per_row) * kRowChunk;
-    const int n = min(kRowChunk, n_outer - t0);
+    const int b = blk / blocks_per_row, t0 = (blk - b * blocks_per_row) * row_chunk;
+    const int n = min(row_chunk, n_outer - t0);
     *first_row = b * n_outer + t0;
     *rows = n;
     const int sum = __reduce_add_sync(0xffffffffu, lane < n ? __ldcg(counts + *first_row + lane) : 0);
@@ -130,7 +130,7 @@ __device__ void launch_order(OrderSmem& sm, const int32_t* counts, int32_t* orde
     pos = __shfl_sync(0xffffffffu, pos, 0);
     pos2 = __shfl_sync(0xffffffffu, pos2, 0);
     if (lane < rows) order[pos + lane] = first + lane;
-    // a block starts at an even tile of its batch row (kRowChunk is even): its pairs are (first + 2j, first + 2j + 1)
+    // a block starts at an even tile of its batch row (the chunk is even): its pairs are (first + 2j, first + 2j + 1)
     if (lane < (rows + 1) / 2) pair_order[pos2 + lane] = first + 2 * lane;
   }
 }
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, 2) schedule_kernel(const __grid_cons
   if (s_last) {
     __threadfence();
     if (a.prefix) list_prefix(s_order.warp_tot, a.counts, a.prefix, a.n_outer_tiles * gridDim.y);
-    else launch_order(s_order, a.counts, a.order, a.pair_order, a.n_outer_tiles, gridDim.y);
+    else launch_order(s_order, a.counts, a.order, a.pair_order, a.n_outer_tiles, gridDim.y, a.row_chunk);
   }
 }
 
