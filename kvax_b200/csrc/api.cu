@@ -299,7 +299,7 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   a.pack = fl.split.pack; a.tile_tokens = fl.split.tile_tokens; a.token_blocks = fl.split.token_blocks; a.head_items = fl.split.head_items;
   a.min_tiles = fl.split.min_tiles;
   a.parts = reinterpret_cast<float*>(ws + fl.parts_off); a.part_ml = reinterpret_cast<float2*>(ws + fl.part_ml_off);
-  a.part_counters = counters + 4;
+  a.part_counters = counters + 5;
   if (fl.split.use) return launch_attn_fwd_split(L, st);
   return pairs ? launch_attn_fwd(L, st) : launch_attn_fwd_one(L, st);
 }
@@ -414,6 +414,7 @@ extern "C" int kvax_b200_attn_bwd(const kvax_b200_attn_bwd_params* p, void* work
   a.q_heads = s.q_heads; a.kv_heads = s.kv_heads; a.group = s.q_heads / s.kv_heads;
   a.batch = s.batch;
   a.head_split = 1; a.dkdv_accumulate = 0;
+  a.work_counter = counters + 4;
 
   if (bl.fused) {
     if (stages & 16) {

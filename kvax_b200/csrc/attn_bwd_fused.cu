@@ -2,7 +2,13 @@
 // five matrix products per tile pair (S, dP, dV, dK, dQ) and one exponential per score, instead
 // of the seven products and two exponentials of the dQ kernel + dK/dV kernel pair in attn_bwd.cu.
 //
-// CTA = (128-row kv tile, kv head, batch); K and V of the tile stay in shared memory; the Q tiles
+// One CTA per SM; a piece of work is (128-row kv tile, kv head, batch) and some or all of the head's query heads, and the
+// producer warp hands the pieces out, longest first.  Rings and barrier phases run on from one piece to the next: the Q and dO
+// of the next piece, its K and V and its first two products come while dK and dV of the last one are stored.  (With a CTA
+// per piece, starting and ending one took 9 of 24 us on 4 x 4k tokens: backward kernel 815 us, now 785; one row of 8k tokens
+// 581 / 570; 8 x 2112 tokens at head_dim 64 184 / 165; the 32k document-mask workload, 390 us a piece, the same.)
+//
+// K and V of the kv tile stay in shared memory; the Q tiles
 // (with the 128 LSE2 / delta values of their queries) of every query head of the GQA group x every
 // listed query tile stream through a two-stage TMA ring, the dO tiles through a single buffer (dO is
 // dead once dV has run, long before the next dP needs its successor).  Fourteen warps:
@@ -40,7 +46,7 @@
 // head_dim 64: the same kernel with the room that is left over: three Q stages, two dO stages, two dS^T tiles, and TMEM
 // T1 | T2 | dV | dK | dQ | dQ with dQ in columns of its own, so that dP^T(i+1) is issued as soon as dS^T(i) is written and
 // nothing waits for the drain but the dQ two items later.  8 x 2112 tokens, 16 heads, fp16, packed: 412 us as the dQ and dK/dV
-// kernel pair, 188 us.
+// kernel pair, 165 us.
 //
 // dQ is accumulated with fp32 atomics at L2, so its summation order (and last bits) vary from run
 // to run; dK and dV are accumulated in TMEM in a fixed order.
@@ -49,6 +55,7 @@
 // and flash_attention_backward_kernel_dkdv (:874-1191); the element mask of partial tiles is the
 // kv-outer rule of :1067-1167.
 #include <cuda_runtime.h>
+#include <limits.h>
 
 #include "attn_common.cuh"
 #include "internal.h"
@@ -87,7 +94,16 @@ constexpr int kSlice = kTile / 2;                      // columns per register-m
 constexpr int kStageBuf = 32 * 32 * 4;                 // one drain staging buffer: 32 rows x 32 fp32
 
 enum FBar { F_XFULL = 0, F_QFULL0, F_QFULL1, F_QFULL2, F_QEMPTY0, F_QEMPTY1, F_QEMPTY2, F_DOFULL0, F_DOFULL1, F_DOEMPTY0,
-            F_DOEMPTY1, F_SFULL, F_PFULL, F_DPFULL, F_DSFULL, F_DQFULL0, F_DQFULL1, F_DRAINED0, F_DRAINED1, F_ACCFULL, F_COUNT };
+            F_DOEMPTY1, F_SFULL, F_PFULL, F_DPFULL, F_DSFULL, F_DQFULL0, F_DQFULL1, F_DRAINED0, F_DRAINED1, F_ACCFULL,
+            F_WFULL0, F_WFULL1, F_WEMPTY0, F_WEMPTY1, F_COUNT };
+constexpr int kSlotReaders = kComputeWarps + kDrainWarps + 1;   // warps that read a work slot
+
+// What the producer tells the other warps about a piece of work: one kv tile and some query heads of its kv head.
+struct WorkSlot {
+  int b, kt, kvh, first_head;   // batch row, kv tile, kv head, first query head
+  int count;                    // query tiles in the list, or -1: no more work
+  int list_row;
+};
 
 // Position in a ring of N buffers, and the parity of the barrier phase its present use belongs to.
 template <int N>
@@ -118,10 +134,10 @@ struct FusedSmem {
   static constexpr int kBars = kCols + kQStages * 2 * kColBytes;
   static constexpr int kTmemSlot = kBars + 8 * F_COUNT;
   static constexpr int kAbort = kTmemSlot + 4;
-  static constexpr int kTotal = kAbort + 4;
+  static constexpr int kSlots = kAbort + 4;                       // two work slots
+  static constexpr int kTotal = kSlots + 2 * int(sizeof(WorkSlot));
   static_assert(kTotal <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
-  // the epilogue's boxes: two per register-math warp and 64 columns, in the buffers between K / V and the drain's staging
-  static_assert(kComputeWarps * (D / 64) * 2 * kStageBuf <= kStage - kQ, "dK / dV boxes do not fit the idle buffers");
+  static_assert(kCols % 16 == 0 && kSlots % 4 == 0, "alignment");
 };
 
 // Mask bits of kv row r for the 64 queries [i0, i0 + 64) of a partial list entry that carries no element mask from the
@@ -160,50 +176,19 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   }
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // With `head_split` > 1 the query heads of a kv head are divided over that many CTAs (short or few lists would
-  // otherwise leave SMs idle behind a few long CTAs); their dK / dV parts meet in fp32 accumulators by atomic adds.
-  int row_rank, hh;
-  decode_block(blockIdx.x, a.list.row_chunk, a.list.n_outer_tiles * a.batch, a.kv_heads * a.head_split, &row_rank, &hh);
-  const int kvh = hh / a.head_split;
-  const long long list_row = __ldg(a.list.order + row_rank);     // longest lists first
-  const int b = int(list_row / a.list.n_outer_tiles), kt = int(list_row % a.list.n_outer_tiles);
-  const int group = a.group / a.head_split;                      // query heads of this CTA
-  const int first_head = kvh * a.group + (hh % a.head_split) * group;
-  const int count = __ldg(a.list.counts + list_row);
-  const uint32_t* list = a.list.tiles + list_row * a.list.n_inner_tiles;
-  const int n_items = count * group;           // item i: query head kvh*group + i / count, query tile list[i % count]
+  // With `head_split` > 1 the query heads of a kv head are divided over that many pieces of work (short or few lists would
+  // otherwise leave SMs idle behind a few long ones); their dK / dV parts meet in fp32 accumulators by atomic adds.
+  const int group = a.group / a.head_split;                      // query heads of a piece of work
   const int q_len = a.tok.q_len;
-
+  WorkSlot* slots = reinterpret_cast<WorkSlot*>(smem + L::kSlots);
   const int row = tid & (kTile - 1);           // kv row / TMEM lane of a register-math thread
   const int half = (tid >> 7) & 1;             // its column half; in the epilogue its half of the D columns
-  const int r = kt * kTile + row;
   const bool is_compute = tid < kComputeThreads;
-  const bool row_valid = is_compute && (r < a.tok.kv_len);
-  // dK / dV rows of this thread: fp32, or 16-bit elements of the operand type when the caller asked for that
-  const long long dkv_off = (((long long)b * a.tok.kv_len + r) * a.kv_heads + kvh) * D + half * (D / 2);
-  float* dk_row = a.dk + dkv_off;
-  float* dv_row = a.dv + dkv_off;
-  uint16_t* dk_row16 = reinterpret_cast<uint16_t*>(a.dk) + dkv_off;
-  uint16_t* dv_row16 = reinterpret_cast<uint16_t*>(a.dv) + dkv_off;
-
-  if (n_items == 0) {                          // no contributing tile: zero gradients (nothing to add to accumulators)
-    if (row_valid && !a.dkdv_accumulate) {
-      if (a.dkdv_16bit) {
-        const uint4 z = make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int i = 0; i < D / 16; ++i) { reinterpret_cast<uint4*>(dk_row16)[i] = z; reinterpret_cast<uint4*>(dv_row16)[i] = z; }
-      } else {
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i) { reinterpret_cast<float4*>(dk_row)[i] = z; reinterpret_cast<float4*>(dv_row)[i] = z; }
-      }
-    }
-    return;
-  }
 
   if (tid == 0) {
     for (int i = 0; i < F_COUNT; ++i) {
-      const int n = (i == F_PFULL || i == F_DSFULL) ? kComputeThreads : ((i == F_DRAINED0 || i == F_DRAINED1) ? kDrainWarps * 32 : 1);
+      const int n = (i == F_PFULL || i == F_DSFULL) ? kComputeThreads : ((i == F_DRAINED0 || i == F_DRAINED1) ? kDrainWarps * 32 :
+                    ((i == F_WEMPTY0 || i == F_WEMPTY1) ? kSlotReaders : 1));
       mbar_init(&bars[i], n);
     }
     *abort_flag = 0;
@@ -216,89 +201,148 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tT1 = tmem_base, tT2 = tmem_base + kTile;
   const uint32_t tDV = tmem_base + 2 * kTile, tDK = tmem_base + 2 * kTile + D;
-  // dQ of item i: over dP^T in T2, or columns of its own, taken in turn
-  auto dq_columns = [&](int i) { return L::kOwnDq ? tDK + D + (i & 1) * D : tT2; };
+  // dQ of tile t: over dP^T in T2, or columns of its own, taken in turn
+  auto dq_columns = [&](int t) { return L::kOwnDq ? tDK + D + (t & 1) * D : tT2; };
+  // Next piece of work, number w of this CTA: waits for the producer's slot; false when there is no more.  Whole warp.  The
+  // slot may be read until it is given back.
+  auto take_work = [&](int w) -> bool {
+    bool got = mbar_wait(&bars[F_WFULL0 + (w & 1)], uint32_t(w >> 1) & 1u, abort_flag, a.status, F_WFULL0 + (w & 1));
+    got = __all_sync(0xffffffffu, got);
+    return got && slots[w & 1].count >= 0;
+  };
+  auto give_back = [&](int w) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars[F_WEMPTY0 + (w & 1)]);
+  };
+  auto work_list = [&](int list_row) { return a.list.tiles + (long long)list_row * a.list.n_inner_tiles; };
 
   if (warp == kProducerWarp) {
     // ------------------------------------------------------------------ producer (whole warp; one elected lane issues)
-    const int n = __shfl_sync(0xffffffffu, n_items, 0);
-    const int cnt = __shfl_sync(0xffffffffu, count, 0);
-    if (elect_one()) {
-      prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_do);
-      mbar_arrive_expect_tx(&bars[F_XFULL], 2 * L::kTileBytes);
-#pragma unroll
-      for (int x = 0; x < D / 64; ++x) {
-        tma_load_4d(smem + L::kX1 + x * L::kBoxBytes, &tmap_k, &bars[F_XFULL], x * 64, kvh, kt * kTile, b);
-        tma_load_4d(smem + L::kX2 + x * L::kBoxBytes, &tmap_v, &bars[F_XFULL], x * 64, kvh, kt * kTile, b);
-      }
-    }
-    __syncwarp();
+    // It also deals out the work: the first piece is the CTA's own number, the others come from a counter, asked for with the
+    // last tile of a piece (asked for a piece ahead, neighbouring tiles no longer run at the same time and the 32k
+    // document-mask workload is 20 % slower: its operands fall out of L2).  The CTA that gets the counter's last value sets it back to zero.
+    if (elect_one()) { prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_do); }
     bool ok = true;
-    uint32_t e_next = __ldg(list);                 // list entries are fetched one iteration ahead
-    int li = 0, qh = first_head;                  // index into the list, query head
+    const int n_rows = a.list.n_outer_tiles * a.batch, head_items = a.kv_heads * a.head_split;
+    const int n_work = n_rows * head_items;
+    int wi = blockIdx.x, t = 0, n_acc = 0;        // number of the work; tiles so far; pieces of work with tiles so far
     Ring<L::kQStages> rq;
     Ring<L::kDoStages> rd;
     PH_BEGIN()
-    for (int i = 0; i < n && ok; ++i) {
-      const int st = rq.st;
-      const int u = int(e_next & a.list.tile_mask);
-      const int yh = qh;
-      if (++li == cnt) { li = 0; ++qh; }
-      if (i + 1 < n) e_next = __ldg(list + li);
-      PH(1)
-      // ---- Q(i) with LSE2 / delta: its stage is free once dK of the item that had it before has completed
-      if (i >= L::kQStages) {
-        ok = mbar_wait(&bars[F_QEMPTY0 + st], rq.ph ^ 1u, abort_flag, a.status, F_QEMPTY0 + st);
+    for (int w = 0; ok; ++w) {
+      WorkSlot s{0, 0, 0, 0, -1, 0};
+      int fetched = 0;
+      if (wi < n_work) {
+        int row_rank, hh;
+        decode_block(wi, a.list.row_chunk, n_rows, head_items, &row_rank, &hh);
+        s.list_row = __ldg(a.list.order + row_rank);                              // longest lists first
+        s.count = __ldg(a.list.counts + s.list_row);
+        s.b = s.list_row / a.list.n_outer_tiles;
+        s.kt = s.list_row - s.b * a.list.n_outer_tiles;
+        s.kvh = hh / a.head_split;
+        s.first_head = s.kvh * a.group + (hh - s.kvh * a.head_split) * group;
+      }
+      if (w >= 2) {
+        ok = mbar_wait(&bars[F_WEMPTY0 + (w & 1)], uint32_t((w >> 1) - 1) & 1u, abort_flag, a.status, F_WEMPTY0 + (w & 1));
         ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
       }
-      PH(0)
-      if (!ok) break;
-      uint8_t* yq = smem + L::kQ + st * L::kTileBytes;
-      float* cs = s_cols + st * 2 * kTile;
-      const int col0 = u * kTile;
-      const float* lse_src = a.lse + ((long long)b * a.q_heads + yh) * q_len + col0;
-      const float* dl_src = a.delta + ((long long)b * a.q_heads + yh) * q_len + col0;
-      const bool bulk = (col0 + kTile <= q_len) &&
-                        (((reinterpret_cast<uintptr_t>(lse_src) | reinterpret_cast<uintptr_t>(dl_src)) & 15) == 0);
-      if (!bulk) {                                 // tile cut by the end of the sequence, or unaligned rows
+      if (lane == 0) {
+        slots[w & 1] = s;
+        mbar_arrive(&bars[F_WFULL0 + (w & 1)]);
+      }
+      __syncwarp();
+      if (s.count < 0) break;
+      const int b = s.b, kvh = s.kvh, cnt = __shfl_sync(0xffffffffu, s.count, 0);
+      const int n = cnt * group;                 // tile i: query head first_head + i / cnt, query tile list[i % cnt]
+      const uint32_t* list = work_list(s.list_row);
+      auto load_kv = [&]() {
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&bars[F_XFULL], 2 * L::kTileBytes);
 #pragma unroll
-        for (int k = 0; k < kTile / 32; ++k) {
-          const int j = lane + 32 * k;
-          const bool valid = col0 + j < q_len;
-          cs[j] = valid ? __ldg(lse_src + j) : INFINITY;            // exp2(-inf) = 0
-          cs[kTile + j] = valid ? __ldg(dl_src + j) : 0.f;
+          for (int x = 0; x < D / 64; ++x) {
+            tma_load_4d(smem + L::kX1 + x * L::kBoxBytes, &tmap_k, &bars[F_XFULL], x * 64, kvh, s.kt * kTile, b);
+            tma_load_4d(smem + L::kX2 + x * L::kBoxBytes, &tmap_v, &bars[F_XFULL], x * 64, kvh, s.kt * kTile, b);
+          }
         }
-        fence_proxy_async_smem();
-      }
-      __syncwarp();
-      if (elect_one()) {
-        mbar_arrive_expect_tx(&bars[F_QFULL0 + st], L::kTileBytes + (bulk ? 2 * L::kColBytes : 0));
+        __syncwarp();
+      };
+      if (n > 0 && n_acc == 0) load_kv();
+      uint32_t e_next = n > 0 ? __ldg(list) : 0u;    // list entries are fetched one iteration ahead
+      int li = 0, qh = s.first_head;                // index into the list, query head
+      for (int i = 0; i < n && ok; ++i, ++t) {
+        const int st = rq.st;
+        const int u = int(e_next & a.list.tile_mask);
+        const int yh = qh;
+        if (++li == cnt) { li = 0; ++qh; }
+        if (i + 1 < n) e_next = __ldg(list + li);
+        else if (lane == 0) fetched = atomicAdd(a.work_counter, 1);
+        PH(1)
+        // ---- Q(t) with LSE2 / delta: its stage is free once dK of the tile that had it before has completed
+        if (t >= L::kQStages) {
+          ok = mbar_wait(&bars[F_QEMPTY0 + st], rq.ph ^ 1u, abort_flag, a.status, F_QEMPTY0 + st);
+          ok = __all_sync(0xffffffffu, ok);
+        }
+        PH(0)
+        if (!ok) break;
+        uint8_t* yq = smem + L::kQ + st * L::kTileBytes;
+        float* cs = s_cols + st * 2 * kTile;
+        const int col0 = u * kTile;
+        const float* lse_src = a.lse + ((long long)b * a.q_heads + yh) * q_len + col0;
+        const float* dl_src = a.delta + ((long long)b * a.q_heads + yh) * q_len + col0;
+        const bool bulk = (col0 + kTile <= q_len) &&
+                          (((reinterpret_cast<uintptr_t>(lse_src) | reinterpret_cast<uintptr_t>(dl_src)) & 15) == 0);
+        if (!bulk) {                                 // tile cut by the end of the sequence, or unaligned rows
 #pragma unroll
-        for (int x = 0; x < D / 64; ++x) tma_load_4d(yq + x * L::kBoxBytes, &tmap_q, &bars[F_QFULL0 + st], x * 64, yh, u * kTile, b);
-        if (bulk) {
-          bulk_load_1d(cs, lse_src, L::kColBytes, &bars[F_QFULL0 + st]);
-          bulk_load_1d(cs + kTile, dl_src, L::kColBytes, &bars[F_QFULL0 + st]);
+          for (int k = 0; k < kTile / 32; ++k) {
+            const int j = lane + 32 * k;
+            const bool valid = col0 + j < q_len;
+            cs[j] = valid ? __ldg(lse_src + j) : INFINITY;            // exp2(-inf) = 0
+            cs[kTile + j] = valid ? __ldg(dl_src + j) : 0.f;
+          }
+          fence_proxy_async_smem();
+        }
+        __syncwarp();
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&bars[F_QFULL0 + st], L::kTileBytes + (bulk ? 2 * L::kColBytes : 0));
+#pragma unroll
+          for (int x = 0; x < D / 64; ++x) tma_load_4d(yq + x * L::kBoxBytes, &tmap_q, &bars[F_QFULL0 + st], x * 64, yh, u * kTile, b);
+          if (bulk) {
+            bulk_load_1d(cs, lse_src, L::kColBytes, &bars[F_QFULL0 + st]);
+            bulk_load_1d(cs + kTile, dl_src, L::kColBytes, &bars[F_QFULL0 + st]);
+          }
+        }
+        __syncwarp();
+        // ---- dO(t): its buffer is free once dV of the tile that had it before has completed
+        if (t >= L::kDoStages) {
+          ok = mbar_wait(&bars[F_DOEMPTY0 + rd.st], rd.ph ^ 1u, abort_flag, a.status, F_DOEMPTY0 + rd.st);
+          ok = __all_sync(0xffffffffu, ok);
+        }
+        PH(2)
+        if (!ok) break;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&bars[F_DOFULL0 + rd.st], L::kTileBytes);
+#pragma unroll
+          for (int x = 0; x < D / 64; ++x)
+            tma_load_4d(smem + L::kDO + rd.st * L::kTileBytes + x * L::kBoxBytes, &tmap_do, &bars[F_DOFULL0 + rd.st], x * 64, yh, u * kTile, b);
+        }
+        __syncwarp();
+        rq.next();
+        rd.next();
+        // K and V of this work behind its first Q and dO: their buffers are free once the products of the work before are done
+        if (i == 0 && n_acc > 0) {
+          ok = mbar_wait(&bars[F_ACCFULL], uint32_t(n_acc - 1) & 1u, abort_flag, a.status, F_ACCFULL);
+          ok = __all_sync(0xffffffffu, ok);
+          if (ok) load_kv();
         }
       }
-      __syncwarp();
-      // ---- dO(i): its buffer is free once dV of the item that had it before has completed
-      if (i >= L::kDoStages) {
-        ok = mbar_wait(&bars[F_DOEMPTY0 + rd.st], rd.ph ^ 1u, abort_flag, a.status, F_DOEMPTY0 + rd.st);
-        ok = __all_sync(0xffffffffu, ok);
-      }
-      PH(2)
-      if (!ok) break;
-      if (elect_one()) {
-        mbar_arrive_expect_tx(&bars[F_DOFULL0 + rd.st], L::kTileBytes);
-#pragma unroll
-        for (int x = 0; x < D / 64; ++x)
-          tma_load_4d(smem + L::kDO + rd.st * L::kTileBytes + x * L::kBoxBytes, &tmap_do, &bars[F_DOFULL0 + rd.st], x * 64, yh, u * kTile, b);
-      }
-      __syncwarp();
-      rq.next();
-      rd.next();
+      if (n > 0) ++n_acc;
+      else if (lane == 0) fetched = atomicAdd(a.work_counter, 1);
+      fetched = __shfl_sync(0xffffffffu, fetched, 0);
+      if (fetched == n_work - 1 && lane == 0) *a.work_counter = 0;
+      wi = int(gridDim.x) + fetched;
     }
-    PH_END(3, n)
+    PH_END(3, t)
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issuer (whole warp; one elected lane issues)
     constexpr uint32_t idesc_t = make_idesc_16(kTile, kTile, 0, 0, kF16);    // X (K-major) x Y (K-major)
@@ -313,7 +357,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     const uint32_t ds_addr = smem_u32(smem + L::kDS);
     const uint32_t ds_mn_lo0 = sdesc_lo_sw128(ds_addr, L::kBoxBytes), ds_k_lo0 = sdesc_lo_sw128(ds_addr, 16);
     constexpr uint32_t kTileStep = L::kTileBytes >> 4, kDsStep = L::kDsBytes >> 4;   // descriptor steps between buffers
-    const int n = __shfl_sync(0xffffffffu, n_items, 0);
     bool ok = true;
     // `tmem_sync`: the barrier orders TMEM loads / stores of other threads before the MMAs that follow; barriers
     // completed by TMA alone need no tcgen05 fence.
@@ -329,23 +372,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         umma_ss_lo(t_addr, x_lo + off, y_lo + off, idesc_t, kk > 0);
       }
     };
-    wait(F_XFULL, 0, false);
-    if (ok) wait(F_QFULL0, 0, false);
-    if (ok) wait(F_DOFULL0, 0, false);
-    if (ok) {
-      if (elect_one()) {
-        issue_t(tT1, x1_lo, sdesc_lo_sw128(qbase, 16));
-        umma_commit(&bars[F_SFULL]);
-        issue_t(tT2, x2_lo, do_k_lo);
-        umma_commit(&bars[F_DPFULL]);
-      }
-      __syncwarp();
-    }
-    Ring<L::kQStages> rq, rqn;                   // buffers of Q(i), Q(i+1)
+    Ring<L::kQStages> rq, rqn;                   // buffers of the present and the next tile's Q
     Ring<L::kDoStages> rd, rdn;
     rqn.next();
     rdn.next();
-    auto issue_dp_next = [&]() {                 // dP^T of item i+1
+    int t = 0, n_acc = 0;
+    auto issue_dp_next = [&]() {                 // dP^T of the next tile
       wait(F_DOFULL0 + rdn.st, rdn.ph, false);
       if (!ok) return;
       if (elect_one()) {
@@ -355,74 +387,98 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
       __syncwarp();
     };
     PH_BEGIN()
-    for (int i = 0; i < n && ok; ++i) {
-      const uint32_t ph = uint32_t(i & 1);
-      const uint32_t yq = qbase + rq.st * L::kTileBytes, yqn = qbase + rqn.st * L::kTileBytes;
-      const uint32_t acc_on = (i > 0) ? 1u : 0u;
-      const bool more = (i + 1 < n);
-      wait(F_PFULL, ph, true);                                                      // P^T(i) written, S^T(i) consumed
-      PH(0)
+    for (int w = 0; ok && take_work(w); ++w) {
+      const int n = __shfl_sync(0xffffffffu, slots[w & 1].count, 0) * group;
+      give_back(w);
+      if (n == 0) continue;
+      wait(F_XFULL, uint32_t(n_acc) & 1u, false);
+      if (ok) wait(F_QFULL0 + rq.st, rq.ph, false);
       if (!ok) break;
       if (elect_one()) {
-        // dV += P^T dO: the half h of the register-math threads wrote its four K-steps at column offset 64 h
-        const uint32_t do_lo = do_n_lo + rd.st * kTileStep;
-#pragma unroll
-        for (int kk = 0; kk < kTile / 16; ++kk)
-          umma_ts_lo(tDV, tT1 + (kk >> 2) * kSlice + (kk & 3) * 8, do_lo + ((kk * 16 * 128) >> 4), idesc_dv, acc_on | (kk > 0));
-        umma_commit(&bars[F_DOEMPTY0 + rd.st]);                                     // dO(i) is dead: its buffer may be refilled
+        issue_t(tT1, x1_lo, sdesc_lo_sw128(qbase + rq.st * L::kTileBytes, 16));
+        umma_commit(&bars[F_SFULL]);
       }
       __syncwarp();
-      PH(1)
-      if (more) {
-        wait(F_QFULL0 + rqn.st, rqn.ph, false);
-        PH(2)
+      if (!L::kOwnDq && t > 0) wait(F_DRAINED0, uint32_t(t - 1) & 1u, true);          // dQ of the last tile has left the T2 columns
+      if (ok) wait(F_DOFULL0 + rd.st, rd.ph, false);
+      if (!ok) break;
+      if (elect_one()) {
+        issue_t(tT2, x2_lo, do_k_lo + rd.st * kTileStep);
+        umma_commit(&bars[F_DPFULL]);
+      }
+      __syncwarp();
+      // the products below overwrite dV and dK of the work before: every register-math thread has read them before it arrives
+      // with its first P^T
+      for (int i = 0; i < n && ok; ++i, ++t) {
+        const uint32_t ph = uint32_t(t & 1);
+        const uint32_t yq = qbase + rq.st * L::kTileBytes, yqn = qbase + rqn.st * L::kTileBytes;
+        const uint32_t acc_on = (i > 0) ? 1u : 0u;
+        const bool more = (i + 1 < n);
+        wait(F_PFULL, ph, true);                                                      // P^T(i) written, S^T(i) consumed
+        PH(0)
         if (!ok) break;
         if (elect_one()) {
-          issue_t(tT1, x1_lo, sdesc_lo_sw128(yqn, 16));                             // scores of item i+1
-          umma_commit(&bars[F_SFULL]);
+          // dV += P^T dO: the half h of the register-math threads wrote its four K-steps at column offset 64 h
+          const uint32_t do_lo = do_n_lo + rd.st * kTileStep;
+#pragma unroll
+          for (int kk = 0; kk < kTile / 16; ++kk)
+            umma_ts_lo(tDV, tT1 + (kk >> 2) * kSlice + (kk & 3) * 8, do_lo + ((kk * 16 * 128) >> 4), idesc_dv, acc_on | (kk > 0));
+          umma_commit(&bars[F_DOEMPTY0 + rd.st]);                                     // dO(i) is dead: its buffer may be refilled
         }
         __syncwarp();
-        PH(3)
-      }
-      wait(F_DSFULL, ph, true);                                                     // dS^T(i) in its tile, dP^T(i) consumed
-      PH(4)
-      if (!ok) break;
-      const uint32_t tdq = dq_columns(i);
-      if (L::kOwnDq) {
-        if (more) issue_dp_next();                                                  // T2 is free already
-        if (ok && i >= 2) wait(F_DRAINED0 + (i & 1), uint32_t((i >> 1) - 1) & 1u, true);   // dQ(i-2) has left its columns
-        if (!ok) break;
-      }
-      if (elect_one()) {
-        const uint32_t ds_off = L::kDsTiles == 2 ? (i & 1) * kDsStep : 0u;
-        const uint32_t ds_mn_lo = ds_mn_lo0 + ds_off, ds_k_lo = ds_k_lo0 + ds_off;
-        // dQ(i) = dS K: both operands read with kv as the contraction index (16 kv rows per step = 16 lines of 128 bytes)
-#pragma unroll
-        for (int kk = 0; kk < kTile / 16; ++kk)
-          umma_ss_lo(tdq, ds_mn_lo + ((kk * 16 * 128) >> 4), kmn_lo + ((kk * 16 * 128) >> 4), idesc_dq, kk > 0);
-        umma_commit(&bars[F_DQFULL0 + (L::kOwnDq ? (i & 1) : 0)]);
-        // dK(i) += dS^T(i) Q(i)
-        const uint32_t q_lo = sdesc_lo_sw128(yq, L::kBoxBytes);
-#pragma unroll
-        for (int kk = 0; kk < kTile / 16; ++kk) {
-          const uint32_t off = ((kk >> 2) * L::kBoxBytes + (kk & 3) * 32) >> 4;
-          umma_ss_lo(tDK, ds_k_lo + off, q_lo + ((kk * 16 * 128) >> 4), idesc_dk, acc_on | (kk > 0));
+        PH(1)
+        if (more) {
+          wait(F_QFULL0 + rqn.st, rqn.ph, false);
+          PH(2)
+          if (!ok) break;
+          if (elect_one()) {
+            issue_t(tT1, x1_lo, sdesc_lo_sw128(yqn, 16));                             // scores of item i+1
+            umma_commit(&bars[F_SFULL]);
+          }
+          __syncwarp();
+          PH(3)
         }
-        umma_commit(&bars[F_QEMPTY0 + rq.st]);                                      // Q(i) is dead; also: the dS^T tile may be rewritten
-        if (!more) umma_commit(&bars[F_ACCFULL]);
-      }
-      __syncwarp();
-      PH(5)
-      if (!L::kOwnDq && more) {
-        wait(F_DRAINED0, ph, true);                                                 // dQ(i) has left the T2 columns
-        PH(6)
-        if (ok) issue_dp_next();
+        wait(F_DSFULL, ph, true);                                                     // dS^T(i) in its tile, dP^T(i) consumed
+        PH(4)
         if (!ok) break;
-        PH(7)
+        const uint32_t tdq = dq_columns(t);
+        if (L::kOwnDq) {
+          if (more) issue_dp_next();                                                  // T2 is free already
+          if (ok && t >= 2) wait(F_DRAINED0 + (t & 1), uint32_t((t >> 1) - 1) & 1u, true);   // the dQ before the last has left its columns
+          if (!ok) break;
+        }
+        if (elect_one()) {
+          const uint32_t ds_off = L::kDsTiles == 2 ? (t & 1) * kDsStep : 0u;
+          const uint32_t ds_mn_lo = ds_mn_lo0 + ds_off, ds_k_lo = ds_k_lo0 + ds_off;
+          // dQ(i) = dS K: both operands read with kv as the contraction index (16 kv rows per step = 16 lines of 128 bytes)
+#pragma unroll
+          for (int kk = 0; kk < kTile / 16; ++kk)
+            umma_ss_lo(tdq, ds_mn_lo + ((kk * 16 * 128) >> 4), kmn_lo + ((kk * 16 * 128) >> 4), idesc_dq, kk > 0);
+          umma_commit(&bars[F_DQFULL0 + (L::kOwnDq ? (t & 1) : 0)]);
+          // dK(i) += dS^T(i) Q(i)
+          const uint32_t q_lo = sdesc_lo_sw128(yq, L::kBoxBytes);
+#pragma unroll
+          for (int kk = 0; kk < kTile / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * L::kBoxBytes + (kk & 3) * 32) >> 4;
+            umma_ss_lo(tDK, ds_k_lo + off, q_lo + ((kk * 16 * 128) >> 4), idesc_dk, acc_on | (kk > 0));
+          }
+          umma_commit(&bars[F_QEMPTY0 + rq.st]);                                      // Q(i) is dead; also: the dS^T tile may be rewritten
+          if (!more) umma_commit(&bars[F_ACCFULL]);
+        }
+        __syncwarp();
+        PH(5)
+        if (!L::kOwnDq && more) {
+          wait(F_DRAINED0, ph, true);                                                 // dQ(i) has left the T2 columns
+          PH(6)
+          if (ok) issue_dp_next();
+          if (!ok) break;
+          PH(7)
+        }
+        rq.next(); rqn.next(); rd.next(); rdn.next();
       }
-      rq.next(); rqn.next(); rd.next(); rdn.next();
+      ++n_acc;
     }
-    PH_END(1, n)
+    PH_END(1, t)
   } else if (is_compute) {
     // ------------------------------------------------------------------ register math
     const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
@@ -430,184 +486,225 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     const uint32_t my_t1 = tT1 + lane_base + cb;              // fp32 columns of this thread; P^T goes to the first 32 of them
     const uint32_t my_t2 = tT2 + lane_base + cb;
     const float c = a.scale_log2e;
-    // Mask bits of this thread's 64 queries of partial list entry e: the element mask the list builder worked out (one
-    // 8-byte load), else computed by the function above.
-    auto item_keep = [&](uint32_t e, uint32_t* k2) {
-      const uint2 w = (e & kBitmapBit) ? __ldg(reinterpret_cast<const uint2*>(entry_bitmap(a.list, e) + row) + half)
-                                       : fused_keep_slow(&a, b, r, int(e & a.list.tile_mask) * kTile + cb);
-      k2[0] = w.x; k2[1] = w.y;
-    };
-
-    bool ok = true;
-    uint32_t e_next = ldg_pinned(list);
-    int li = 0;
-    // mask bits of the coming item are fetched one item ahead (in the gap while dP^T of the current item is
-    // awaited), so that their global loads never sit in front of the exponentials
-    uint32_t keep_next[2] = {0xffffffffu, 0xffffffffu};
-    if (e_next & kPartialBit) item_keep(e_next, keep_next);
     uint8_t* ds_row = smem + L::kDS + half * (kTile * 128) + row * 128;  // this thread's 128-byte row of the dS^T tile
-    Ring<L::kQStages> rq, rfree;                            // buffer of Q(i); of the last item that read the tile dS^T(i) goes to
+    Ring<L::kQStages> rq, rfree;                            // buffer of Q(t); of the last tile that read the buffer dS^T(t) goes to
+    bool ok = true;
+    int t = 0, n_acc = 0;
     PH_BEGIN()
-    for (int i = 0; i < n_items && ok; ++i) {
-      const uint32_t e = e_next;
-      if (++li == count) li = 0;
-      if (i + 1 < n_items) e_next = ldg_pinned(list + li);
-      const bool partial = (e & kPartialBit) != 0;
-      const int st = rq.st;
-      const uint32_t ph = uint32_t(i & 1);
-      const float* cs = s_cols + st * 2 * kTile;
-      const float4* cs_lse = reinterpret_cast<const float4*>(cs + cb);
-      const float4* cs_dl = reinterpret_cast<const float4*>(cs + kTile + cb);
-      const uint32_t keep[2] = {keep_next[0], keep_next[1]};
-
-      // LSE2 / delta of this item have landed together with its Q tile
-      ok = mbar_wait(&bars[F_QFULL0 + st], rq.ph, abort_flag, a.status, F_QFULL0 + st);
-      rq.next();
-      PH(1)
-      if (!ok) break;
-
-      // ---- A: P^T = exp2(S^T * scale*log2e - LSE2); the 64 values of this thread stay in registers for B
-      ok = mbar_wait(&bars[F_SFULL], ph, abort_flag, a.status, F_SFULL);
-      PH(2)
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t v[2][32];
-      tmem_ld32(my_t1, v[0]);
-      tmem_ld32(my_t1 + 32, v[1]);
-#pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {
-        tmem_ld_wait(v[ch]);
-#pragma unroll
-        for (int jj = 0; jj < 32; jj += 4) {
-          const float4 ls = cs_lse[(ch * 32 + jj) >> 2];
-          const float l4[4] = {ls.x, ls.y, ls.z, ls.w};
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            float pv = fast_exp2(fmaf(__uint_as_float(v[ch][jj + t]), c, -l4[t]));
-            if (partial) pv = ((keep[ch] >> (jj + t)) & 1u) ? pv : 0.f;
-            v[ch][jj + t] = __float_as_uint(pv);
-          }
+    for (int w = 0; ok && take_work(w); ++w) {
+      // read where it is needed, so that it lives in no register of the tile loop
+      const volatile WorkSlot& s = slots[w & 1];
+      const int count = s.count, n_items = count * group;
+      const uint32_t* list = work_list(s.list_row);
+      // dK / dV rows of this thread: fp32, or 16-bit elements of the operand type when the caller asked for that
+      auto dkv_offset = [&]() {
+        return (((long long)s.b * a.tok.kv_len + s.kt * kTile + row) * a.kv_heads + s.kvh) * D + half * (D / 2);
+      };
+      if (n_items == 0) {                          // no contributing tile: zero gradients (nothing to add to accumulators)
+        if (s.kt * kTile + row < a.tok.kv_len && !a.dkdv_accumulate) {
+          const long long dkv_off = dkv_offset();
+          const int n_vec = D / 2 * (a.dkdv_16bit ? 2 : 4) / 16;
+          uint4* zk = a.dkdv_16bit ? reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.dk) + dkv_off) : reinterpret_cast<uint4*>(a.dk + dkv_off);
+          uint4* zv = a.dkdv_16bit ? reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.dv) + dkv_off) : reinterpret_cast<uint4*>(a.dv + dkv_off);
+          for (int i = 0; i < n_vec; ++i) { zk[i] = make_uint4(0, 0, 0, 0); zv[i] = make_uint4(0, 0, 0, 0); }
         }
-        uint32_t pk[16];
-#pragma unroll
-        for (int jj = 0; jj < 32; jj += 2) pk[jj >> 1] = pack16<kF16>(__uint_as_float(v[ch][jj]), __uint_as_float(v[ch][jj + 1]));
-        tmem_st16(my_t1 + ch * 16, pk);
+        give_back(w);
+        continue;
       }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars[F_PFULL]);
-      PH(3)
+      // Mask bits of this thread's 64 queries of partial list entry e: the element mask the list builder worked out (one
+      // 8-byte load), else computed by the function above.
+      auto item_keep = [&](uint32_t e, uint32_t* k2) {
+        const uint2 m = (e & kBitmapBit) ? __ldg(reinterpret_cast<const uint2*>(entry_bitmap(a.list, e) + row) + half)
+                                         : fused_keep_slow(&a, s.b, s.kt * kTile + row, int(e & a.list.tile_mask) * kTile + cb);
+        k2[0] = m.x; k2[1] = m.y;
+      };
+      uint32_t e_next = ldg_pinned(list);
+      int li = 0;
+      // mask bits of the coming tile are fetched one tile ahead (in the gap while dP^T of the current one is
+      // awaited), so that their global loads never sit in front of the exponentials
+      uint32_t keep_next[2] = {0xffffffffu, 0xffffffffu};
+      if (e_next & kPartialBit) item_keep(e_next, keep_next);
+      for (int i = 0; i < n_items && ok; ++i, ++t) {
+        const uint32_t e = e_next;
+        if (++li == count) li = 0;
+        if (i + 1 < n_items) e_next = ldg_pinned(list + li);
+        const bool partial = (e & kPartialBit) != 0;
+        const int st = rq.st;
+        const uint32_t ph = uint32_t(t & 1);
+        const float* cs = s_cols + st * 2 * kTile;
+        const float4* cs_lse = reinterpret_cast<const float4*>(cs + cb);
+        const float4* cs_dl = reinterpret_cast<const float4*>(cs + kTile + cb);
+        const uint32_t keep[2] = {keep_next[0], keep_next[1]};
 
-      keep_next[0] = keep_next[1] = 0xffffffffu;
-      if (i + 1 < n_items && (e_next & kPartialBit)) item_keep(e_next, keep_next);
-      PH(0)
-
-      // ---- B: dS^T = P^T * (dP^T - delta) -> bf16 -> the dS^T tile in shared memory
-      ok = mbar_wait(&bars[F_DPFULL], ph, abort_flag, a.status, F_DPFULL);
-      PH(4)
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t dp[2][16];                                     // 16 columns at a time, the next request in flight
-      tmem_ld16(my_t2, dp[0]);
-      if (i >= L::kDsTiles) {      // dQ and dK of the tile's last item have completed (the commit that frees that item's Q stage)
-        ok = mbar_wait(&bars[F_QEMPTY0 + rfree.st], rfree.ph, abort_flag, a.status, F_QEMPTY0 + rfree.st);
-        rfree.next();
+        // LSE2 / delta of this item have landed together with its Q tile
+        ok = mbar_wait(&bars[F_QFULL0 + st], rq.ph, abort_flag, a.status, F_QFULL0 + st);
+        rq.next();
+        PH(1)
         if (!ok) break;
-      }
-      PH(5)
-      {
-        // kv row `row`, queries [64 half, 64 half + 64) = one 128-byte row of box `half`: eight 16-byte chunks at the
-        // positions the 128-byte swizzle assigns them
-        uint8_t* slot = ds_row + (L::kDsTiles == 2 ? (i & 1) * L::kDsBytes : 0);
-#pragma unroll
-        for (int sc = 0; sc < 4; ++sc) {                      // columns [16 sc, 16 sc + 16) of this thread's 64
-          if (sc + 1 < 4) tmem_ld16(my_t2 + (sc + 1) * 16, dp[(sc + 1) & 1]);
-          tmem_ld_wait16(dp[sc & 1]);
-          const int ch = sc >> 1, j0 = (sc & 1) * 16;
-#pragma unroll
-          for (int jj = 0; jj < 16; jj += 8) {
-            const float4 dl0 = cs_dl[(sc * 16 + jj) >> 2], dl1 = cs_dl[((sc * 16 + jj) >> 2) + 1];
-            const float dl[8] = {dl0.x, dl0.y, dl0.z, dl0.w, dl1.x, dl1.y, dl1.z, dl1.w};
-            float d[8];
-#pragma unroll
-            for (int t = 0; t < 8; ++t)
-              d[t] = __uint_as_float(v[ch][j0 + jj + t]) * (__uint_as_float(dp[sc & 1][jj + t]) - dl[t]);
-            const int ck = sc * 2 + (jj >> 3);                // 16-byte chunk: 8 queries
-            *reinterpret_cast<uint4*>(slot + ((ck ^ (row & 7)) << 4)) =
-                make_uint4(pack16<kF16>(d[0], d[1]), pack16<kF16>(d[2], d[3]), pack16<kF16>(d[4], d[5]), pack16<kF16>(d[6], d[7]));
-          }
-        }
-      }
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(&bars[F_DSFULL]);
-      PH(6)
-    }
-    if (warp == 0) { PH_END(0, n_items) }
 
-    if (ok) ok = mbar_wait(&bars[F_ACCFULL], 0, abort_flag, a.status, F_ACCFULL);
-    if (ok) {
-      tc_fence_after();
-      // every thread stores D/2 columns of its row: columns [half*D/2, (half+1)*D/2)
+        // ---- A: P^T = exp2(S^T * scale*log2e - LSE2); the 64 values of this thread stay in registers for B
+        ok = mbar_wait(&bars[F_SFULL], ph, abort_flag, a.status, F_SFULL);
+        PH(2)
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t v[2][32];
+        tmem_ld32(my_t1, v[0]);
+        tmem_ld32(my_t1 + 32, v[1]);
 #pragma unroll
-      for (int ch = 0; ch < D / 64; ++ch) {
-        uint32_t v1[32], v2[32];
-        tmem_ld32(tDV + lane_base + half * (D / 2) + ch * 32, v1);
-        tmem_ld32(tDK + lane_base + half * (D / 2) + ch * 32, v2);
-        tmem_ld_wait(v1);
-        tmem_ld_wait(v2);
-        if (a.dkdv_accumulate) {
-          // Parts of several CTAs meet in fp32 accumulators: the warp's 32 x 32 boxes go through shared memory (the Q, dO and dS^T
-          // buffers are idle by now) and are added by TMA.  (Reductions straight from registers, a row per lane, ran at half
-          // the rate: 5900 clk for 128 x 128 floats per SM, measured alone, against 2800 for whole 128-byte lines.)
-          uint8_t* box = smem + L::kQ + ((warp * (D / 64) + ch) * 2) * kStageBuf;
-          auto put = [&](uint8_t* dst, const uint32_t (&x)[32], float f) {
+        for (int ch = 0; ch < 2; ++ch) {
+          tmem_ld_wait(v[ch]);
 #pragma unroll
-            for (int ck = 0; ck < 8; ++ck)
-              *reinterpret_cast<float4*>(dst + lane * 128 + ((ck ^ (lane & 7)) << 4)) =
-                  make_float4(__uint_as_float(x[4 * ck]) * f, __uint_as_float(x[4 * ck + 1]) * f, __uint_as_float(x[4 * ck + 2]) * f,
-                              __uint_as_float(x[4 * ck + 3]) * f);
-          };
-          put(box, v1, 1.f);
-          put(box + kStageBuf, v2, a.scale);
-          fence_proxy_async_smem();
-          __syncwarp();
-          const int r0 = kt * kTile + (warp & 3) * 32, col = half * (D / 2) + ch * 32;
-          if (lane == 0 && r0 < a.tok.kv_len) {               // rows beyond the sequence are clipped by TMA
-            tma_reduce_add_4d(&tmap_dv, box, col, kvh, r0, b);
-            tma_reduce_add_4d(&tmap_dk, box + kStageBuf, col, kvh, r0, b);
-            bulk_commit_group();
-          }
-        } else if (row_valid) {
-          if (a.dkdv_16bit) {
+          for (int jj = 0; jj < 32; jj += 4) {
+            const float4 ls = cs_lse[(ch * 32 + jj) >> 2];
+            const float l4[4] = {ls.x, ls.y, ls.z, ls.w};
 #pragma unroll
-            for (int jj = 0; jj < 32; jj += 8) {
-              uint4 w1, w2;
-              w1.x = pack16<kF16>(__uint_as_float(v1[jj + 0]), __uint_as_float(v1[jj + 1]));
-              w1.y = pack16<kF16>(__uint_as_float(v1[jj + 2]), __uint_as_float(v1[jj + 3]));
-              w1.z = pack16<kF16>(__uint_as_float(v1[jj + 4]), __uint_as_float(v1[jj + 5]));
-              w1.w = pack16<kF16>(__uint_as_float(v1[jj + 6]), __uint_as_float(v1[jj + 7]));
-              w2.x = pack16<kF16>(__uint_as_float(v2[jj + 0]) * a.scale, __uint_as_float(v2[jj + 1]) * a.scale);
-              w2.y = pack16<kF16>(__uint_as_float(v2[jj + 2]) * a.scale, __uint_as_float(v2[jj + 3]) * a.scale);
-              w2.z = pack16<kF16>(__uint_as_float(v2[jj + 4]) * a.scale, __uint_as_float(v2[jj + 5]) * a.scale);
-              w2.w = pack16<kF16>(__uint_as_float(v2[jj + 6]) * a.scale, __uint_as_float(v2[jj + 7]) * a.scale);
-              reinterpret_cast<uint4*>(dv_row16)[(ch * 32 + jj) >> 3] = w1;
-              reinterpret_cast<uint4*>(dk_row16)[(ch * 32 + jj) >> 3] = w2;
+            for (int t = 0; t < 4; ++t) {
+              float pv = fast_exp2(fmaf(__uint_as_float(v[ch][jj + t]), c, -l4[t]));
+              if (partial) pv = ((keep[ch] >> (jj + t)) & 1u) ? pv : 0.f;
+              v[ch][jj + t] = __float_as_uint(pv);
             }
-          } else {
+          }
+          uint32_t pk[16];
 #pragma unroll
-            for (int jj = 0; jj < 32; jj += 4) {
-              reinterpret_cast<float4*>(dv_row)[(ch * 32 + jj) >> 2] =
-                  make_float4(__uint_as_float(v1[jj]), __uint_as_float(v1[jj + 1]), __uint_as_float(v1[jj + 2]), __uint_as_float(v1[jj + 3]));
-              reinterpret_cast<float4*>(dk_row)[(ch * 32 + jj) >> 2] =
-                  make_float4(__uint_as_float(v2[jj]) * a.scale, __uint_as_float(v2[jj + 1]) * a.scale,
-                              __uint_as_float(v2[jj + 2]) * a.scale, __uint_as_float(v2[jj + 3]) * a.scale);
+          for (int jj = 0; jj < 32; jj += 2) pk[jj >> 1] = pack16<kF16>(__uint_as_float(v[ch][jj]), __uint_as_float(v[ch][jj + 1]));
+          tmem_st16(my_t1 + ch * 16, pk);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&bars[F_PFULL]);
+        PH(3)
+
+        keep_next[0] = keep_next[1] = 0xffffffffu;
+        if (i + 1 < n_items && (e_next & kPartialBit)) item_keep(e_next, keep_next);
+        PH(0)
+
+        // ---- B: dS^T = P^T * (dP^T - delta) -> bf16 -> the dS^T tile in shared memory
+        ok = mbar_wait(&bars[F_DPFULL], ph, abort_flag, a.status, F_DPFULL);
+        PH(4)
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t dp[2][16];                                     // 16 columns at a time, the next request in flight
+        tmem_ld16(my_t2, dp[0]);
+        if (t >= L::kDsTiles) {      // dQ and dK of the buffer's last tile have completed (the commit that frees that tile's Q stage)
+          ok = mbar_wait(&bars[F_QEMPTY0 + rfree.st], rfree.ph, abort_flag, a.status, F_QEMPTY0 + rfree.st);
+          rfree.next();
+          if (!ok) break;
+        }
+        PH(5)
+        {
+          // kv row `row`, queries [64 half, 64 half + 64) = one 128-byte row of box `half`: eight 16-byte chunks at the
+          // positions the 128-byte swizzle assigns them
+          uint8_t* slot = ds_row + (L::kDsTiles == 2 ? (t & 1) * L::kDsBytes : 0);
+#pragma unroll
+          for (int sc = 0; sc < 4; ++sc) {                      // columns [16 sc, 16 sc + 16) of this thread's 64
+            if (sc + 1 < 4) tmem_ld16(my_t2 + (sc + 1) * 16, dp[(sc + 1) & 1]);
+            tmem_ld_wait16(dp[sc & 1]);
+            const int ch = sc >> 1, j0 = (sc & 1) * 16;
+#pragma unroll
+            for (int jj = 0; jj < 16; jj += 8) {
+              const float4 dl0 = cs_dl[(sc * 16 + jj) >> 2], dl1 = cs_dl[((sc * 16 + jj) >> 2) + 1];
+              const float dl[8] = {dl0.x, dl0.y, dl0.z, dl0.w, dl1.x, dl1.y, dl1.z, dl1.w};
+              float d[8];
+#pragma unroll
+              for (int t = 0; t < 8; ++t)
+                d[t] = __uint_as_float(v[ch][j0 + jj + t]) * (__uint_as_float(dp[sc & 1][jj + t]) - dl[t]);
+              const int ck = sc * 2 + (jj >> 3);                // 16-byte chunk: 8 queries
+              *reinterpret_cast<uint4*>(slot + ((ck ^ (row & 7)) << 4)) =
+                  make_uint4(pack16<kF16>(d[0], d[1]), pack16<kF16>(d[2], d[3]), pack16<kF16>(d[4], d[5]), pack16<kF16>(d[6], d[7]));
+            }
+          }
+        }
+        fence_proxy_async_smem();
+        tc_fence_before();
+        mbar_arrive(&bars[F_DSFULL]);
+        PH(6)
+      }
+
+      // ---- dV and dK of the work: the products of the next one may start meanwhile (scores and dP^T only)
+      if (ok) ok = mbar_wait(&bars[F_ACCFULL], uint32_t(n_acc) & 1u, abort_flag, a.status, F_ACCFULL);
+      ok = __all_sync(0xffffffffu, ok);
+      ++n_acc;
+      if (ok) {
+        tc_fence_after();
+        const int b = s.b, kvh = s.kvh;
+        const bool row_valid = s.kt * kTile + row < a.tok.kv_len;
+        const long long dkv_off = dkv_offset();
+        float* dk_row = a.dk + dkv_off;
+        float* dv_row = a.dv + dkv_off;
+        uint16_t* dk_row16 = reinterpret_cast<uint16_t*>(a.dk) + dkv_off;
+        uint16_t* dv_row16 = reinterpret_cast<uint16_t*>(a.dv) + dkv_off;
+        // every thread stores D/2 columns of its row: columns [half*D/2, (half+1)*D/2)
+#pragma unroll 1
+        for (int ch = 0; ch < D / 64; ++ch) {
+          uint32_t v1[32], v2[32];
+          tmem_ld32(tDV + lane_base + half * (D / 2) + ch * 32, v1);
+          tmem_ld32(tDK + lane_base + half * (D / 2) + ch * 32, v2);
+          tmem_ld_wait(v1);
+          tmem_ld_wait(v2);
+          if (a.dkdv_accumulate) {
+            // Parts of several CTAs meet in fp32 accumulators: the warp's 32 x 32 boxes go through its own 4 KB of the dS^T
+            // tile(s) -- whose readers are done, and which only this warp writes -- and are added by TMA.  (Reductions straight
+            // from registers, a row per lane, ran at half the rate: 5900 clk for 128 x 128 floats per SM, measured alone,
+            // against 2800 for whole 128-byte lines.)
+            const int r0 = s.kt * kTile + (warp & 3) * 32, col = half * (D / 2) + ch * 32;
+            uint8_t* box = smem + L::kDS + half * (kTile * 128) + (warp & 3) * kStageBuf;
+            auto add = [&](const void* tmap, uint8_t* dst, const uint32_t (&x)[32], float f) {
+#pragma unroll
+              for (int ck = 0; ck < 8; ++ck)
+                *reinterpret_cast<float4*>(dst + lane * 128 + ((ck ^ (lane & 7)) << 4)) =
+                    make_float4(__uint_as_float(x[4 * ck]) * f, __uint_as_float(x[4 * ck + 1]) * f, __uint_as_float(x[4 * ck + 2]) * f,
+                                __uint_as_float(x[4 * ck + 3]) * f);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                if (r0 < a.tok.kv_len) tma_reduce_add_4d(tmap, dst, col, kvh, r0, b);       // rows beyond the sequence are clipped by TMA
+                bulk_commit_group();
+              }
+            };
+            auto box_free = [&]() {
+              if (lane == 0) bulk_wait_group_read<0>();
+              __syncwarp();
+            };
+            if (ch > 0) box_free();
+            add(&tmap_dv, box, v1, 1.f);
+            if (L::kDsTiles == 1) box_free();
+            add(&tmap_dk, box + (L::kDsTiles - 1) * L::kDsBytes, v2, a.scale);
+          } else if (row_valid) {
+            if (a.dkdv_16bit) {
+#pragma unroll
+              for (int jj = 0; jj < 32; jj += 8) {
+                uint4 w1, w2;
+                w1.x = pack16<kF16>(__uint_as_float(v1[jj + 0]), __uint_as_float(v1[jj + 1]));
+                w1.y = pack16<kF16>(__uint_as_float(v1[jj + 2]), __uint_as_float(v1[jj + 3]));
+                w1.z = pack16<kF16>(__uint_as_float(v1[jj + 4]), __uint_as_float(v1[jj + 5]));
+                w1.w = pack16<kF16>(__uint_as_float(v1[jj + 6]), __uint_as_float(v1[jj + 7]));
+                w2.x = pack16<kF16>(__uint_as_float(v2[jj + 0]) * a.scale, __uint_as_float(v2[jj + 1]) * a.scale);
+                w2.y = pack16<kF16>(__uint_as_float(v2[jj + 2]) * a.scale, __uint_as_float(v2[jj + 3]) * a.scale);
+                w2.z = pack16<kF16>(__uint_as_float(v2[jj + 4]) * a.scale, __uint_as_float(v2[jj + 5]) * a.scale);
+                w2.w = pack16<kF16>(__uint_as_float(v2[jj + 6]) * a.scale, __uint_as_float(v2[jj + 7]) * a.scale);
+                reinterpret_cast<uint4*>(dv_row16)[(ch * 32 + jj) >> 3] = w1;
+                reinterpret_cast<uint4*>(dk_row16)[(ch * 32 + jj) >> 3] = w2;
+              }
+            } else {
+#pragma unroll
+              for (int jj = 0; jj < 32; jj += 4) {
+                reinterpret_cast<float4*>(dv_row)[(ch * 32 + jj) >> 2] =
+                    make_float4(__uint_as_float(v1[jj]), __uint_as_float(v1[jj + 1]), __uint_as_float(v1[jj + 2]), __uint_as_float(v1[jj + 3]));
+                reinterpret_cast<float4*>(dk_row)[(ch * 32 + jj) >> 2] =
+                    make_float4(__uint_as_float(v2[jj]) * a.scale, __uint_as_float(v2[jj + 1]) * a.scale,
+                                __uint_as_float(v2[jj + 2]) * a.scale, __uint_as_float(v2[jj + 3]) * a.scale);
+              }
             }
           }
         }
       }
+      if (ok && a.dkdv_accumulate) {                            // the dS^T tile may be written again
+        if (lane == 0) bulk_wait_group_read<0>();
+      }
+      give_back(w);
     }
-    if (a.dkdv_accumulate && lane == 0) bulk_wait_group<0>();  // performed before the CTA goes away
+    if (warp == 0) { PH_END(0, t) }
+    if (lane == 0) bulk_wait_group<0>();                      // all reduce-adds performed before the CTA goes away
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ dQ drain (warps 8-11)
@@ -617,78 +714,85 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     uint8_t* my_row = stage + lane * 128;                     // this lane's query row in staging buffer 0: 32 fp32, swizzled
     if (lane == 0) prefetch_tmap(&tmap_dq);
     bool ok = true;
-    uint32_t e_next = ldg_pinned(list);
-    int li = 0, qh = first_head;
+    int t = 0;
     PH_BEGIN()
-    for (int i = 0; i < n_items && ok; ++i) {
-      const int q0 = int(e_next & a.list.tile_mask) * kTile + dw * 32;    // first query row this warp drains
-      const int yh = qh;
-      if (++li == count) { li = 0; ++qh; }
-      if (i + 1 < n_items) e_next = ldg_pinned(list + li);
-      const bool live = q0 < q_len;                           // rows beyond the sequence are clipped by TMA; skip all-out boxes
-      const int db = L::kOwnDq ? (i & 1) : 0;
-      const uint32_t tdq = dq_columns(i) + lane_base;
-      ok = mbar_wait(&bars[F_DQFULL0 + db], uint32_t(L::kOwnDq ? (i >> 1) : i) & 1u, abort_flag, a.status, F_DQFULL0 + db);
-      PH(0)
-      if (!ok) break;
-      tc_fence_after();
-      // Registers hold three 32-column chunks at a time (the register file leaves 128 per thread): chunks 0-2 are
-      // requested at once; chunk 0 is written to its staging buffer as soon as it arrives and chunk 3 is requested
-      // into its registers right behind those stores; the T2 columns are released as soon as all chunks are in
-      // registers, and everything else (proxy fence, reduce-add, the other chunks) happens after that.
-      auto put = [&](int ch, const uint32_t (&x)[32]) {       // registers -> staging buffer ch & 1
-        uint8_t* dst = my_row + (ch & 1) * kStageBuf;
+    for (int w = 0; ok && take_work(w); ++w) {
+      const volatile WorkSlot& s = slots[w & 1];                // read where it is needed, so that it lives in no register
+      const int n_items = s.count * group;
+      const uint32_t* list = work_list(s.list_row);
+      uint32_t e_next = n_items > 0 ? ldg_pinned(list) : 0u;
+      int li = 0, qh = s.first_head;
+      for (int i = 0; i < n_items && ok; ++i, ++t) {
+        const int q0 = int(e_next & a.list.tile_mask) * kTile + dw * 32;    // first query row this warp drains
+        const int yh = qh;
+        if (++li == s.count) { li = 0; ++qh; }
+        if (i + 1 < n_items) e_next = ldg_pinned(list + li);
+        const bool live = q0 < q_len;                           // rows beyond the sequence are clipped by TMA; skip all-out boxes
+        const int db = L::kOwnDq ? (t & 1) : 0;
+        const uint32_t tdq = dq_columns(t) + lane_base;
+        ok = mbar_wait(&bars[F_DQFULL0 + db], uint32_t(L::kOwnDq ? (t >> 1) : t) & 1u, abort_flag, a.status, F_DQFULL0 + db);
+        PH(0)
+        if (!ok) break;
+        tc_fence_after();
+        // Registers hold three 32-column chunks at a time (the register file leaves 128 per thread): chunks 0-2 are
+        // requested at once; chunk 0 is written to its staging buffer as soon as it arrives and chunk 3 is requested
+        // into its registers right behind those stores; the T2 columns are released as soon as all chunks are in
+        // registers, and everything else (proxy fence, reduce-add, the other chunks) happens after that.
+        auto put = [&](int ch, const uint32_t (&x)[32]) {       // registers -> staging buffer ch & 1
+          uint8_t* dst = my_row + (ch & 1) * kStageBuf;
 #pragma unroll
-        for (int ck = 0; ck < 8; ++ck)
-          *reinterpret_cast<uint4*>(dst + ((ck ^ (lane & 7)) << 4)) = make_uint4(x[4 * ck], x[4 * ck + 1], x[4 * ck + 2], x[4 * ck + 3]);
-      };
-      auto reduce = [&](int ch) {                             // staging buffer ch & 1 -> += accumulator
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (live) tma_reduce_add_4d(&tmap_dq, stage + (ch & 1) * kStageBuf, ch * 32, yh, q0, b);
-          // a group is committed for skipped boxes too (it is empty and complete at once): `buffer_free` counts groups,
-          // and a skipped one must not let the group before it, which may still read the other buffer, fall out of the count
-          bulk_commit_group();
+          for (int ck = 0; ck < 8; ++ck)
+            *reinterpret_cast<uint4*>(dst + ((ck ^ (lane & 7)) << 4)) = make_uint4(x[4 * ck], x[4 * ck + 1], x[4 * ck + 2], x[4 * ck + 3]);
+        };
+        auto reduce = [&](int ch) {                             // staging buffer ch & 1 -> += accumulator
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (live) tma_reduce_add_4d(&tmap_dq, stage + (ch & 1) * kStageBuf, ch * 32, yh, q0, s.b);
+            // a group is committed for skipped boxes too (it is empty and complete at once): `buffer_free` counts groups,
+            // and a skipped one must not let the group before it, which may still read the other buffer, fall out of the count
+            bulk_commit_group();
+          }
+        };
+        auto buffer_free = [&]() {                              // the reduce-add issued from the buffer two chunks ago has read it
+          if (lane == 0) bulk_wait_group_read<1>();
+          __syncwarp();
+        };
+        uint32_t x0[32], x1[32];
+        tmem_ld32(tdq, x0);
+        tmem_ld32(tdq + 32, x1);
+        if constexpr (D == 128) {
+          uint32_t x2[32];
+          tmem_ld32(tdq + 64, x2);
+          buffer_free();                                        // buffer 0: chunk 2 of the previous item, long gone
+          tmem_ld_wait(x0);
+          put(0, x0);
+          tmem_ld32(tdq + 96, x0);                              // chunk 3 takes the registers of chunk 0
+          tmem_ld_wait(x1);
+          tmem_ld_wait(x2);
+          tmem_ld_wait(x0);
+          tc_fence_before();
+          mbar_arrive(&bars[F_DRAINED0]);                       // the T2 columns may take dP^T(i+1)
+          PH(1)
+          reduce(0);
+          buffer_free(); put(1, x1); reduce(1);
+          buffer_free(); put(2, x2); reduce(2);
+          buffer_free(); put(3, x0); reduce(3);
+        } else {
+          static_assert(D == 64 || D == 128, "two or four 32-column chunks");
+          tmem_ld_wait(x0);
+          tmem_ld_wait(x1);
+          tc_fence_before();
+          mbar_arrive(&bars[F_DRAINED0 + db]);                  // these columns may take dQ(i+2)
+          PH(1)
+          buffer_free(); put(0, x0); reduce(0);
+          buffer_free(); put(1, x1); reduce(1);
         }
-      };
-      auto buffer_free = [&]() {                              // the reduce-add issued from the buffer two chunks ago has read it
-        if (lane == 0) bulk_wait_group_read<1>();
-        __syncwarp();
-      };
-      uint32_t x0[32], x1[32];
-      tmem_ld32(tdq, x0);
-      tmem_ld32(tdq + 32, x1);
-      if constexpr (D == 128) {
-        uint32_t x2[32];
-        tmem_ld32(tdq + 64, x2);
-        buffer_free();                                        // buffer 0: chunk 2 of the previous item, long gone
-        tmem_ld_wait(x0);
-        put(0, x0);
-        tmem_ld32(tdq + 96, x0);                              // chunk 3 takes the registers of chunk 0
-        tmem_ld_wait(x1);
-        tmem_ld_wait(x2);
-        tmem_ld_wait(x0);
-        tc_fence_before();
-        mbar_arrive(&bars[F_DRAINED0]);                       // the T2 columns may take dP^T(i+1)
-        PH(1)
-        reduce(0);
-        buffer_free(); put(1, x1); reduce(1);
-        buffer_free(); put(2, x2); reduce(2);
-        buffer_free(); put(3, x0); reduce(3);
-      } else {
-        static_assert(D == 64 || D == 128, "two or four 32-column chunks");
-        tmem_ld_wait(x0);
-        tmem_ld_wait(x1);
-        tc_fence_before();
-        mbar_arrive(&bars[F_DRAINED0 + db]);                  // these columns may take dQ(i+2)
-        PH(1)
-        buffer_free(); put(0, x0); reduce(0);
-        buffer_free(); put(1, x1); reduce(1);
+        PH(2)
       }
-      PH(2)
+      give_back(w);
     }
-    if (dw == 0) { PH_END(2, n_items) }
+    if (dw == 0) { PH_END(2, t) }
     if (lane == 0) bulk_wait_group<0>();                      // all reduce-adds performed before the CTA goes away
     __syncwarp();
   }
@@ -734,7 +838,9 @@ int launch_fused(const FusedBwdLaunch& L, cudaStream_t stream) {
   constexpr int smem = FusedSmem<D>::kTotal;
   auto kern = attn_bwd_fused_kernel<D, kF16>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return KVAX_B200_ELAUNCH;
-  dim3 grid(L.args.list.n_outer_tiles * L.batch * L.args.kv_heads * L.args.head_split, 1, 1);
+  const long long work = (long long)L.args.list.n_outer_tiles * L.batch * L.args.kv_heads * L.args.head_split;
+  if (work > INT_MAX - 1024) return KVAX_B200_EUNSUPPORTED;
+  dim3 grid(int(work < kPersistentCtas ? work : kPersistentCtas), 1, 1);
   kern<<<grid, kThreads, smem, stream>>>(L.tmap_k, L.tmap_v, L.tmap_q, L.tmap_do, L.tmap_dq, L.tmap_dk, L.tmap_dv, L.args);
   return cudaGetLastError() == cudaSuccess ? KVAX_B200_OK : KVAX_B200_ELAUNCH;
 }

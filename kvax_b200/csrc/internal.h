@@ -11,7 +11,9 @@ namespace kvx {
 
 constexpr int kSplitCtas = 148;    // forward with the work split over the SMs: one CTA per SM,
 constexpr int kSplitMinTiles = 4;  // none with a smaller share than this (start-up would outweigh it)
-constexpr int kListCounters = 4 + kSplitCtas;   // two per list of a call (the backward builds up to two), one per CTA of the split forward
+constexpr int kPersistentCtas = 148;   // kernels that deal out their work themselves: one CTA per SM
+// two per list of a call (the backward builds up to two), one for dealing out work, one per CTA of the split forward
+constexpr int kListCounters = 5 + kSplitCtas;
 
 struct ScheduleArgs {
   MaskView mask;
@@ -78,6 +80,7 @@ struct BwdArgs {
   float* dv;
   int32_t dkdv_16bit;
   int32_t dkdv_accumulate;  // fused kernel: dk / dv are fp32 accumulators (zero on entry) that every CTA adds its part to
+  int32_t* work_counter;    // fused kernel: pieces of work dealt out beyond the first of every CTA; zero between launches
   int32_t head_split;       // fused kernel: CTAs per (kv tile, kv head), each with group / head_split query heads
   int32_t* status;
   long long dq_strides[3];  // element strides (batch, seq, head) of dq
