@@ -158,7 +158,7 @@ class _ToOperand(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         inv = ctx.box.inv
-        if ctx.in_dtype == torch.float32 and g.dtype in (torch.float16, torch.bfloat16) and g.is_contiguous() and g.numel():
+        if g.is_cuda and ctx.in_dtype == torch.float32 and g.dtype in (torch.float16, torch.bfloat16) and g.is_contiguous() and g.numel():
             out = torch.empty_like(g, dtype=torch.float32)
             with torch.cuda.device(g.device):
                 rc = _lib.load().kvax_b200_widen_to_float(g.data_ptr(), g.numel(), _lib.DTYPE_F16 if g.dtype == torch.float16 else _lib.DTYPE_BF16,
@@ -183,6 +183,10 @@ class _FromOperand(torch.autograd.Function):
         if ctx.op_dtype != torch.float16:
             return g.to(ctx.op_dtype), None, None
         # largest magnitude -> [1, 2): small gradients keep their bits, nothing overflows; exact (power of two)
+        if not g.is_cuda:                        # the same steps on the host
+            s = torch.exp2(-torch.floor(torch.log2(g.abs().amax().clamp_min(1e-30))))
+            ctx.box.inv = 1.0 / s
+            return (g * s).to(torch.float16), None, None
         g = g.contiguous()
         amax = _abs_max(g)
         out = torch.empty_like(g, dtype=torch.float16)
