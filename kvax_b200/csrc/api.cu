@@ -300,6 +300,7 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   a.min_tiles = fl.split.min_tiles;
   a.parts = reinterpret_cast<float*>(ws + fl.parts_off); a.part_ml = reinterpret_cast<float2*>(ws + fl.part_ml_off);
   a.part_counters = counters + 5;
+  a.work_counter = counters + 4;
   if (fl.split.use) return launch_attn_fwd_split(L, st);
   return pairs ? launch_attn_fwd(L, st) : launch_attn_fwd_one(L, st);
 }

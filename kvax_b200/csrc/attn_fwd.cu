@@ -1,6 +1,11 @@
 // Flash-attention forward for sm_100a (B200).
 //
-// One CTA per (head, PAIR of neighbouring 128-row query tiles, batch), one CTA per SM, eleven warps:
+// A piece of work is a PAIR of neighbouring 128-row query tiles of one head, or one query tile of two heads of a kv group
+// (grouped-query attention).  One CTA per SM; the K producer hands the pieces out, longest first, and rings and barrier phases
+// run on: the first K, Q and scores of the next piece come while a group still stores its tile of the last one.  (A CTA per
+// piece spent 8 of 26 us on starting and ending one on 4 x 4k tokens.  With that, masks of partial tiles applied in one block
+// and their fallback out of line: 4 x 4k tokens 371 -> 342 us, 8k 266 -> 251, 2 x 5003 304 -> 279, 2 x 32k documents 3.92 -> 3.77 ms.)
+// Eleven warps:
 //   warps 0-3  softmax group 0: query tile 2p.
 //   warps 4-7  softmax group 1: query tile 2p + 1.
 //              In both groups thread t owns query row (t % 128) = TMEM lane of its tile.  Each group has its
@@ -30,7 +35,10 @@
 // 137-370): scores scaled by scale*log2(e), exp2-domain online softmax, P rounded to the
 // input dtype before P V, O = acc / l, LSE2 = m + log2(l); query tiles with no work get
 // O = 0 and LSE2 = 0 (:253-258).
+#include <limits.h>
+
 #include "attn_common.cuh"
+#include "attn_fwd_mask.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -62,14 +70,23 @@ constexpr int kTmemCols = 512;
 constexpr int kKStages = 3, kVStages = 2;
 
 enum FwdBar {
-  B_QFULL0 = 0, B_QFULL1,
+  B_QFULL0 = 0, B_QFULL1, B_QEMPTY0, B_QEMPTY1,
   B_KFULL0, B_KFULL1, B_KFULL2, B_KEMPTY0, B_KEMPTY1, B_KEMPTY2,
   B_VFULL0, B_VFULL1, B_VEMPTY0, B_VEMPTY1,
   B_SFULL0, B_SFULL1,                        // scores of group g's next list entry are in TMEM
   B_PFULL0, B_PFULL1,                        // kv columns 0-63 of group g's P are in TMEM
   B_PREST0, B_PREST1,                        // kv columns 64-127 too
-  B_DONE0, B_DONE1,                          // the last P V of group g has completed: completes once
+  B_DONE0, B_DONE1,                          // the last P V of group g in a piece of work has completed: completes once per piece
+  B_WFULL0, B_WFULL1, B_WEMPTY0, B_WEMPTY1,  // work slots
   B_COUNT
+};
+constexpr int kSlotReaders = kSoftmaxThreads / 32 + 2;   // warps that read a work slot: softmax, MMA issuer, V producer
+
+// What the K producer tells the other warps about a piece of work: two work items that share their K / V tiles.
+struct WorkSlot {
+  int row0;              // list row of item 0
+  int head;              // head, or pair of heads
+  int n0, n1;            // list lengths; n0 = -1: no more work
 };
 
 template <int D>
@@ -83,7 +100,8 @@ struct FwdSmem {
   static constexpr int kTmemSlot = kBars + 8 * B_COUNT;
   static constexpr int kAbort = kTmemSlot + 4;
   static constexpr int kDesc = kAbort + 4;             // one word per K stage: what the MMA issuer does with the entry
-  static constexpr int kTotal = kDesc + 4 * kKStages + 1024;   // + slack for 1024-byte alignment
+  static constexpr int kSlots = kDesc + 4 * kKStages;          // two work slots
+  static constexpr int kTotal = kSlots + 2 * int(sizeof(WorkSlot)) + 1024;   // + slack for 1024-byte alignment
   static_assert(kTotal <= 232448, "exceeds the 227 KB of shared memory a CTA may use");
 };
 
@@ -127,11 +145,12 @@ constexpr uint32_t kDescMore = 4u;                        // there is an entry u
 constexpr uint32_t kDescN0 = 8u, kDescN1 = 16u;           // ... in the list of tile 0 / tile 1
 constexpr uint32_t kDescLast1 = 32u;                      // ... whose scores group 1 issues last (else group 0)
 constexpr uint32_t kDescFin0 = 64u, kDescFin1 = 128u;     // entry u is the last one of tile 0 / tile 1
+constexpr uint32_t kDescNFin0 = 256u, kDescNFin1 = 512u;  // entry u + 1 is
 
 template <int D, bool kF16>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                const __grid_constant__ CUtensorMap tmap_v, const FwdArgs a) {
+                const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FwdArgs a) {
   using L = FwdSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -149,40 +168,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   // grouped-query attention -- one query tile of two query heads that read the same kv head: then both items have
   // the same tile list, every K / V tile serves both and no union entry is ever one-sided.
   const int ph = a.pair_heads ? 1 : 0;
-  int pair_rank, hh;
-  decode_block(blockIdx.x, a.list.row_chunk, (ph ? n_outer : (n_outer + 1) / 2) * a.batch, ph ? a.q_heads / 2 : a.q_heads, &pair_rank, &hh);
-  const long long row0 = __ldg((ph ? a.list.order : a.list.pair_order) + pair_rank);     // list row of item 0
-  const int b = int(row0 / n_outer), qt0 = int(row0 % n_outer);
-  const bool has1 = ph || qt0 + 1 < n_outer;
-  const int h0 = ph ? 2 * hh : hh;                       // query head of item 0; item 1: h0 + ph
-  const int kvh = h0 / a.group;
-  const int n0 = __ldg(a.list.counts + row0);
-  const int n1 = ph ? n0 : (has1 ? __ldg(a.list.counts + row0 + 1) : 0);
-  const uint32_t* list0 = a.list.tiles + row0 * a.list.n_inner_tiles;
-  const uint32_t* list1 = ph ? list0 : list0 + a.list.n_inner_tiles;
+  const uint32_t n_lists = uint32_t(ph ? n_outer : (n_outer + 1) / 2) * a.batch, head_items = ph ? a.q_heads / 2 : a.q_heads;
+  WorkSlot* slots = reinterpret_cast<WorkSlot*>(smem + L::kSlots);
 
   const int row = tid & (kTile - 1);
-  const int wg = (tid >> 7) & 1;                         // softmax group = work item of the CTA
-  const int qt = qt0 + (ph ? 0 : wg);
-  const int h = h0 + (ph ? wg : 0);                      // query head of this thread's item
-  const int r = qt * kTile + row;                        // query row of a softmax thread
-  const bool is_softmax = tid < kSoftmaxThreads;
-  const bool row_valid = is_softmax && (r < a.tok.q_len);
-  const int count = wg ? n1 : n0;                        // list length of this thread's tile
-  const uint32_t* list = wg ? list1 : list0;
-  __nv_bfloat16* o_row = a.out + (long long)b * a.o_strides[0] + (long long)r * a.o_strides[1] + (long long)h * a.o_strides[2];
-  float* lse_row = a.lse + ((long long)b * a.q_heads + h) * a.tok.q_len + r;
-
-  if (is_softmax && count == 0 && row_valid) {           // nothing to attend: zeros (:253-258)
-    const uint4 z = make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(o_row)[i] = z;
-    *lse_row = a.empty_lse;
-  }
-  if (n0 == 0 && n1 == 0) return;
+  const int wg = (tid >> 7) & 1;                         // softmax group = work item of the piece
 
   if (tid == 0) {
-    for (int i = 0; i < B_COUNT; ++i) mbar_init(&bars[i], (i >= B_PFULL0 && i <= B_PREST1) ? kTile : 1);
+    for (int i = 0; i < B_COUNT; ++i)
+      mbar_init(&bars[i], (i >= B_PFULL0 && i <= B_PREST1) ? kTile : ((i == B_WEMPTY0 || i == B_WEMPTY1) ? kSlotReaders : 1));
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -192,68 +186,115 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;                 // scores of group g: tmem_base + 128 g
   const uint32_t tO = tmem_base + 2 * kTile;             // accumulator of group g: tO + 128 g
+  // Piece of work number w of this CTA: waits for its slot; false when there is no more.  The slot is given back once read.
+  auto take_work = [&](int w) -> bool {
+    return mbar_wait(&bars[B_WFULL0 + (w & 1)], uint32_t(w >> 1) & 1u, abort_flag, a.status, B_WFULL0 + (w & 1)) && slots[w & 1].n0 >= 0;
+  };
+  auto list_of = [&](int list_row) { return a.list.tiles + (long long)list_row * a.list.n_inner_tiles; };
+  auto second_list = [&](int row0) { return list_of(ph ? row0 : row0 + 1); };
 
   if (warp == kKWarp) {
     // ------------------------------------------------------------------ Q and K producer
+    // It also deals out the work: the first piece is the CTA's own number, the others come from a counter, asked for with the
+    // last K tile of a piece (earlier, neighbouring tiles would no longer run at the same time and share K / V in L2).  The
+    // CTA that gets the counter's last value sets it back to zero.
     if (lane == 0) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k);
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        if ((g ? n1 : n0) == 0) continue;
-        mbar_arrive_expect_tx(&bars[B_QFULL0 + g], L::kTileBytes);
-#pragma unroll
-        for (int x = 0; x < D / 64; ++x)
-          tma_load_4d(sQ + g * L::kTileBytes + x * L::kBoxBytes, &tmap_q, &bars[B_QFULL0 + g], x * 64, h0 + (ph ? g : 0),
-                      (qt0 + (ph ? 0 : g)) * kTile, b);
-      }
-      PairWalk w;
-      w.init(list0, n0, list1, n1, a.list.tile_mask);
+      const int n_work = int(n_lists * head_items);
       bool ok = true;
-      for (int u = 0; w.more() && ok; ++u) {
-        int tile; bool m0, m1;
-        w.next(&tile, &m0, &m1);
-        const int st = u % kKStages, use = u / kKStages;
-        uint32_t desc = (m0 ? kDescM0 : 0u) | (m1 ? kDescM1 : 0u);
-        if (m0 && w.i0 == w.n0) desc |= kDescFin0;
-        if (m1 && w.i1 == w.n1) desc |= kDescFin1;
-        if (w.more()) {
-          bool x0, x1;
-          w.peek(&x0, &x1);
-          desc |= kDescMore | (x0 ? kDescN0 : 0u) | (x1 ? kDescN1 : 0u);
-          // scores of entry u + 1 are issued by the members of entry u first (in group order), then by the rest
-          int last_g = -1;
-          if (x0 && m0) last_g = 0;
-          if (x1 && m1) last_g = 1;
-          if (x0 && !m0) last_g = 0;
-          if (x1 && !m1) last_g = 1;
-          if (last_g == 1) desc |= kDescLast1;
+      int wi = blockIdx.x, u = 0, done0 = 0, done1 = 0;    // number of the work; K tiles so far; pieces with item 0 / 1 so far
+      for (int w = 0; ok; ++w) {
+        WorkSlot s{0, 0, -1, 0};
+        if (wi < n_work) {
+          int pair_rank;
+          decode_block(wi, a.list.row_chunk, int(n_lists), int(head_items), &pair_rank, &s.head);
+          s.row0 = __ldg((ph ? a.list.order : a.list.pair_order) + pair_rank);
+          s.n0 = __ldg(a.list.counts + s.row0);
+          s.n1 = ph ? s.n0 : ((s.row0 % n_outer) + 1 < n_outer ? __ldg(a.list.counts + s.row0 + 1) : 0);
         }
-        if (use > 0) ok = mbar_wait(&bars[B_KEMPTY0 + st], (use - 1) & 1, abort_flag, a.status, B_KEMPTY0 + st);
+        if (w >= 2) ok = mbar_wait(&bars[B_WEMPTY0 + (w & 1)], uint32_t((w >> 1) - 1) & 1u, abort_flag, a.status, B_WEMPTY0 + (w & 1));
         if (!ok) break;
-        step_desc[st] = desc;                                   // published by the arrive below
-        mbar_arrive_expect_tx(&bars[B_KFULL0 + st], L::kTileBytes);
+        slots[w & 1] = s;
+        mbar_arrive(&bars[B_WFULL0 + (w & 1)]);
+        if (s.n0 < 0) break;
+        const int b = s.row0 / n_outer, qt0 = s.row0 - b * n_outer;
+        const int h0 = ph ? 2 * s.head : s.head, kvh = h0 / a.group;
+        PairWalk pw;
+        pw.init(list_of(s.row0), s.n0, second_list(s.row0), s.n1, a.list.tile_mask);
+        int fetched = 0;
+        if (!pw.more()) fetched = atomicAdd(a.work_counter, 1);
+        for (bool first = true; pw.more() && ok; ++u, first = false) {
+          int tile; bool m0, m1;
+          pw.next(&tile, &m0, &m1);
+          const int st = u % kKStages, use = u / kKStages;
+          uint32_t desc = (m0 ? kDescM0 : 0u) | (m1 ? kDescM1 : 0u);
+          if (m0 && pw.i0 == pw.n0) desc |= kDescFin0;
+          if (m1 && pw.i1 == pw.n1) desc |= kDescFin1;
+          if (pw.more()) {
+            bool x0, x1;
+            pw.peek(&x0, &x1);
+            desc |= kDescMore | (x0 ? kDescN0 : 0u) | (x1 ? kDescN1 : 0u);
+            if (x0 && pw.i0 + 1 == pw.n0) desc |= kDescNFin0;
+            if (x1 && pw.i1 + 1 == pw.n1) desc |= kDescNFin1;
+            // scores of entry u + 1 are issued by the members of entry u first (in group order), then by the rest
+            int last_g = -1;
+            if (x0 && m0) last_g = 0;
+            if (x1 && m1) last_g = 1;
+            if (x0 && !m0) last_g = 0;
+            if (x1 && !m1) last_g = 1;
+            if (last_g == 1) desc |= kDescLast1;
+          } else {
+            fetched = atomicAdd(a.work_counter, 1);
+          }
+          if (use > 0) ok = mbar_wait(&bars[B_KEMPTY0 + st], (use - 1) & 1, abort_flag, a.status, B_KEMPTY0 + st);
+          if (!ok) break;
+          step_desc[st] = desc;                                   // published by the arrive below
+          mbar_arrive_expect_tx(&bars[B_KFULL0 + st], L::kTileBytes);
 #pragma unroll
-        for (int x = 0; x < D / 64; ++x)
-          tma_load_4d(sK + st * L::kTileBytes + x * L::kBoxBytes, &tmap_k, &bars[B_KFULL0 + st], x * 64, kvh, tile * kTile, b);
+          for (int x = 0; x < D / 64; ++x)
+            tma_load_4d(sK + st * L::kTileBytes + x * L::kBoxBytes, &tmap_k, &bars[B_KFULL0 + st], x * 64, kvh, tile * kTile, b);
+          if (!first) continue;
+          // the Q tiles behind the first K tile: their buffers are free once the last scores of the piece before are done
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            if ((g ? s.n1 : s.n0) == 0) continue;
+            const int done = g ? done1++ : done0++;
+            if (done > 0) ok = ok && mbar_wait(&bars[B_QEMPTY0 + g], uint32_t(done - 1) & 1u, abort_flag, a.status, B_QEMPTY0 + g);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&bars[B_QFULL0 + g], L::kTileBytes);
+#pragma unroll
+            for (int x = 0; x < D / 64; ++x)
+              tma_load_4d(sQ + g * L::kTileBytes + x * L::kBoxBytes, &tmap_q, &bars[B_QFULL0 + g], x * 64, h0 + (ph ? g : 0),
+                          (qt0 + (ph ? 0 : g)) * kTile, b);
+          }
+        }
+        if (fetched == n_work - 1) *a.work_counter = 0;
+        wi = int(gridDim.x) + fetched;
       }
     }
   } else if (warp == kVWarp) {
     // ------------------------------------------------------------------ V producer
     if (lane == 0) {
       prefetch_tmap(&tmap_v);
-      PairWalk w;
-      w.init(list0, n0, list1, n1, a.list.tile_mask);
       bool ok = true;
-      for (int u = 0; w.more() && ok; ++u) {
-        int tile; bool m0, m1;
-        w.next(&tile, &m0, &m1);
-        const int st = u % kVStages, use = u / kVStages;
-        if (use > 0) ok = mbar_wait(&bars[B_VEMPTY0 + st], (use - 1) & 1, abort_flag, a.status, B_VEMPTY0 + st);
-        if (!ok) break;
-        mbar_arrive_expect_tx(&bars[B_VFULL0 + st], L::kTileBytes);
+      int u = 0;
+      for (int w = 0; ok && take_work(w); ++w) {
+        const WorkSlot s = slots[w & 1];
+        mbar_arrive(&bars[B_WEMPTY0 + (w & 1)]);
+        const int b = s.row0 / n_outer, kvh = (ph ? 2 * s.head : s.head) / a.group;
+        PairWalk pw;
+        pw.init(list_of(s.row0), s.n0, second_list(s.row0), s.n1, a.list.tile_mask);
+        for (; pw.more() && ok; ++u) {
+          int tile; bool m0, m1;
+          pw.next(&tile, &m0, &m1);
+          const int st = u % kVStages, use = u / kVStages;
+          if (use > 0) ok = mbar_wait(&bars[B_VEMPTY0 + st], (use - 1) & 1, abort_flag, a.status, B_VEMPTY0 + st);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&bars[B_VFULL0 + st], L::kTileBytes);
 #pragma unroll
-        for (int x = 0; x < D / 64; ++x)
-          tma_load_4d(sV + st * L::kTileBytes + x * L::kBoxBytes, &tmap_v, &bars[B_VFULL0 + st], x * 64, kvh, tile * kTile, b);
+          for (int x = 0; x < D / 64; ++x)
+            tma_load_4d(sV + st * L::kTileBytes + x * L::kBoxBytes, &tmap_v, &bars[B_VFULL0 + st], x * 64, kvh, tile * kTile, b);
+        }
       }
     }
   } else if (warp == kMmaWarp) {
@@ -261,7 +302,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     constexpr uint32_t idesc_s = make_idesc_16(kTile, kTile, 0, 0, kF16);   // Q (K-major) x K (K-major)
     constexpr uint32_t idesc_o = make_idesc_16(kTile, D, 0, 1, kF16);       // P (TMEM)    x V (N-major)
     const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-    const int cnt0 = __shfl_sync(0xffffffffu, n0, 0), cnt1 = __shfl_sync(0xffffffffu, n1, 0);
     bool ok = true;
     FPH_BEGIN()
     // `tmem_sync`: the barrier orders TMEM loads / stores of other threads before the MMAs that follow; barriers
@@ -272,7 +312,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (tmem_sync) tc_fence_after();
     };
     uint32_t ph0 = 0, ph1 = 0;               // phase of group g's P barriers = number of its P V products so far, mod 2
-    uint32_t acc0 = 0, acc1 = 0;             // group g's accumulator holds something
+    uint32_t q0 = 0, q1 = 0;                 // phase of group g's Q barrier
     uint32_t d_next = 0;                     // descriptor of the entry whose K stage was waited for last
     // K stage of union entry u: waits for the tile and fetches the entry's descriptor
     auto wait_k = [&](int u) {
@@ -282,8 +322,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       d_next = step_desc[st];
       FPH(0)
     };
-    // scores of group g for union entry u; `last`: no other group will read this K stage afterwards
-    auto issue_qk = [&](int g, int u, bool last) {
+    // scores of group g for union entry u; `last`: no other group will read this K stage afterwards; `fin`: the group's last
+    auto issue_qk = [&](int g, int u, bool last, bool fin) {
       const int st = u % kKStages;
       const uint32_t ts = tmem_base + g * kTile;
       const uint32_t q_lo = sdesc_lo_sw128(q_addr + g * L::kTileBytes, 16);
@@ -296,6 +336,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         umma_commit(&bars[B_SFULL0 + g]);
         if (last) umma_commit(&bars[B_KEMPTY0 + st]);     // the K producer may refill the stage
+        if (fin) umma_commit(&bars[B_QEMPTY0 + g]);       // ... and the Q tile
       }
       __syncwarp();
       FPH(1)
@@ -329,45 +370,57 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       __syncwarp();
       FPH(5)
     };
-    if (cnt0 > 0) wait(B_QFULL0, 0, false);
-    if (ok && cnt1 > 0) wait(B_QFULL1, 0, false);
-    if (ok) wait_k(0);
-    uint32_t d = d_next;
-    if (ok && (d & kDescM0)) issue_qk(0, 0, !(d & kDescM1));
-    if (ok && (d & kDescM1)) issue_qk(1, 0, true);
-    int n_pv = 0;
-    for (int u = 0; ok; ++u) {
-      const int vs = u % kVStages, vuse = u / kVStages;
-      const bool more = (d & kDescMore) != 0;
-      const bool last1 = (d & kDescLast1) != 0;
-      FPH(6)
-      wait(B_VFULL0 + vs, vuse & 1, false);
-      FPH(2)
+    int n_pv = 0, u = 0;                     // products so far; union entries so far
+    for (int w = 0; ok; ++w) {
+      bool some = take_work(w);
+      some = __all_sync(0xffffffffu, some);
+      if (!some) break;
+      const int n0 = __shfl_sync(0xffffffffu, slots[w & 1].n0, 0), n1 = __shfl_sync(0xffffffffu, slots[w & 1].n1, 0);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[B_WEMPTY0 + (w & 1)]);
+      if (n0 == 0 && n1 == 0) continue;
+      wait_k(u);
+      if (ok && n0 > 0) { wait(B_QFULL0, q0, false); q0 ^= 1u; }
+      if (ok && n1 > 0) { wait(B_QFULL1, q1, false); q1 ^= 1u; }
       if (!ok) break;
-      bool k_ready = false;
-      if (d & kDescM0) {
-        issue_pv(0, vs, ph0, acc0, !(d & kDescM1), (d & kDescFin0) != 0);
+      uint32_t acc0 = 0, acc1 = 0;           // group g's accumulator holds something
+      uint32_t d = d_next;
+      // these overwrite the scores (and P) of the piece before: its last products were issued before them
+      if (d & kDescM0) issue_qk(0, u, !(d & kDescM1), n0 == 1);
+      if (d & kDescM1) issue_qk(1, u, true, n1 == 1);
+      for (; ok; ++u) {
+        const int vs = u % kVStages, vuse = u / kVStages;
+        const bool more = (d & kDescMore) != 0;
+        const bool last1 = (d & kDescLast1) != 0, nfin0 = (d & kDescNFin0) != 0, nfin1 = (d & kDescNFin1) != 0;
+        FPH(6)
+        wait(B_VFULL0 + vs, vuse & 1, false);
+        FPH(2)
         if (!ok) break;
-        ph0 ^= 1u; acc0 = 1u; ++n_pv;
-        if (more && (d & kDescN0)) {              // reuses S_0: issued after PV(0, u), which read P_0
-          if (!k_ready) { wait_k(u + 1); k_ready = true; if (!ok) break; }
-          issue_qk(0, u + 1, !last1);
+        bool k_ready = false;
+        if (d & kDescM0) {
+          issue_pv(0, vs, ph0, acc0, !(d & kDescM1), (d & kDescFin0) != 0);
+          if (!ok) break;
+          ph0 ^= 1u; acc0 = 1u; ++n_pv;
+          if (more && (d & kDescN0)) {              // reuses S_0: issued after PV(0, u), which read P_0
+            if (!k_ready) { wait_k(u + 1); k_ready = true; if (!ok) break; }
+            issue_qk(0, u + 1, !last1, nfin0);
+          }
         }
-      }
-      if (d & kDescM1) {
-        issue_pv(1, vs, ph1, acc1, true, (d & kDescFin1) != 0);
-        if (!ok) break;
-        ph1 ^= 1u; acc1 = 1u; ++n_pv;
-        if (more && (d & kDescN1)) {
-          if (!k_ready) { wait_k(u + 1); k_ready = true; if (!ok) break; }
-          issue_qk(1, u + 1, last1);
+        if (d & kDescM1) {
+          issue_pv(1, vs, ph1, acc1, true, (d & kDescFin1) != 0);
+          if (!ok) break;
+          ph1 ^= 1u; acc1 = 1u; ++n_pv;
+          if (more && (d & kDescN1)) {
+            if (!k_ready) { wait_k(u + 1); k_ready = true; if (!ok) break; }
+            issue_qk(1, u + 1, last1, nfin1);
+          }
         }
+        if (!more) { ++u; break; }
+        if (!k_ready) { wait_k(u + 1); if (!ok) break; }
+        if ((d & kDescN0) && !(d & kDescM0)) issue_qk(0, u + 1, !last1, nfin0);
+        if ((d & kDescN1) && !(d & kDescM1)) issue_qk(1, u + 1, last1, nfin1);
+        d = d_next;
       }
-      if (!more) break;
-      if (!k_ready) { wait_k(u + 1); if (!ok) break; }
-      if ((d & kDescN0) && !(d & kDescM0)) issue_qk(0, u + 1, !last1);
-      if ((d & kDescN1) && !(d & kDescM1)) issue_qk(1, u + 1, last1);
-      d = d_next;
     }
     FPH_END(2, n_pv)
   } else {
@@ -376,154 +429,161 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t tS = tmem_base + wg * kTile + lane_base;
     const uint32_t tOg = tO + wg * kTile + lane_base;
     const float c = a.scale_log2e;
-    RowBounds rb = load_bounds(a.mask, b, min(r, a.tok.q_len - 1));
-    int q_seg = KVAX_B200_PADDING_SEGMENT_ID, q_pos = 0;
-    if (row_valid) {
-      q_seg = __ldg(a.tok.q_seg + (long long)b * a.tok.q_len + r);
-      q_pos = query_position(a.tok, b, r);
-    }
-    const int32_t* kv_seg = a.tok.kv_seg + (long long)b * a.tok.kv_len;
-    const int32_t* kv_pos = a.tok.kv_pos + (long long)b * a.tok.kv_len;
-
-    // Online softmax state of this group.  `m` is the reference maximum the exponentials
-    // use.  It only follows the true running maximum when that has grown by more than kLazy
-    // (log2 units): P then stays below 2^kLazy and the accumulator in TMEM needs no rescaling
-    // for small increases.
     constexpr float kLazy = 8.f;
-    float m = -INFINITY, l = 0.f;
     bool ok = true;
-    uint32_t e_next = (count > 0) ? ldg_pinned(list) : 0u;     // list entries are fetched one iteration ahead
+    int tiles = 0, pieces = 0;               // score tiles and pieces of work of this group so far
     FPH_BEGIN()
-    for (int it = 0; it < count && ok; ++it) {
-      const uint32_t e = e_next;
-      if (it + 1 < count) e_next = ldg_pinned(list + it + 1);
-      const int c0 = int(e & a.list.tile_mask) * kTile;
-      const bool partial = (e & kPartialBit) != 0;
+    for (int w = 0; ok; ++w) {
+      bool some = take_work(w);
+      some = __all_sync(0xffffffffu, some);
+      if (!some) break;
+      const WorkSlot s = slots[w & 1];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[B_WEMPTY0 + (w & 1)]);
+      const int b = s.row0 / n_outer, qt = s.row0 - b * n_outer + (ph ? 0 : wg);
+      const int h = ph ? 2 * s.head + wg : s.head;             // query head of this group's item
+      const int count = wg ? s.n1 : s.n0;
+      const uint32_t* list = wg ? second_list(s.row0) : list_of(s.row0);
+      const int r = qt * kTile + row;                          // query row of this thread
+      const bool row_valid = qt < n_outer && r < a.tok.q_len;
+      __nv_bfloat16* o_row = a.out + (long long)b * a.o_strides[0] + (long long)r * a.o_strides[1] + (long long)h * a.o_strides[2];
+      float* lse_row = a.lse + ((long long)b * a.q_heads + h) * a.tok.q_len + r;
+      if (count == 0) {                                        // nothing to attend: zeros (:253-258)
+        if (row_valid) {
+          const uint4 z = make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(o_row)[i] = z;
+          *lse_row = a.empty_lse;
+        }
+        continue;
+      }
+      // Online softmax state of this group.  `m` is the reference maximum the exponentials
+      // use.  It only follows the true running maximum when that has grown by more than kLazy
+      // (log2 units): P then stays below 2^kLazy and the accumulator in TMEM needs no rescaling
+      // for small increases.
+      float m = -INFINITY, l = 0.f;
+      uint32_t e_next = ldg_pinned(list);                        // list entries are fetched one iteration ahead
+      for (int it = 0; it < count && ok; ++it, ++tiles) {
+        const uint32_t e = e_next;
+        if (it + 1 < count) e_next = ldg_pinned(list + it + 1);
+        const bool partial = (e & kPartialBit) != 0;
 
-      // element mask of partial tiles (computed before the scores arrive)
-      uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-      if (partial) {
-        if (e & kBitmapBit) {                   // worked out once by the list builder for every head: 16 bytes per row
-          const uint4 w = __ldg(entry_bitmap(a.list, e) + row);
-          keep[0] = w.x; keep[1] = w.y; keep[2] = w.z; keep[3] = w.w;
-        } else {
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch)
-            keep[ch] = keep_bits32<false>(rb, c0 + ch * 32, a.tok.kv_len, row_valid, q_seg, q_pos, kv_seg + c0 + ch * 32,
-                                          a.tok.sequential ? nullptr : kv_pos + c0 + ch * 32);
-        }
-      }
+        // element mask of partial tiles (fetched before the scores arrive): worked out once by the list builder for every head,
+        // 16 bytes per row
+        uint4 keep = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        if (partial) keep = fwd_keep(a, e, b, r, row);
 
-      FPH(0)
-      ok = mbar_wait(&bars[B_SFULL0 + wg], it & 1, abort_flag, a.status, B_SFULL0 + wg);
-      ok = __all_sync(0xffffffffu, ok);         // the warp leaves the loop together (warp-wide votes below)
-      FPH(1)
-      if (!ok) break;
-      tc_fence_after();
-
-      // All 128 scores of the row are read into registers with four back-to-back TMEM loads
-      // (one round trip), reduced to the row maximum, exponentiated in place and written back
-      // as P (bf16 pairs) over the first 64 score columns.
-      uint32_t v[4][32];
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) tmem_ld32(tS + ch * 32, v[ch]);
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // independent chains: no serial dependency
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        tmem_ld_wait(v[ch]);
-        if (partial) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[ch][j] = ((keep[ch] >> j) & 1u) ? v[ch][j] : 0xff800000u;   // -inf
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-#pragma unroll
-          for (int t = 0; t < 4; ++t)
-            mx4[t] = fmax3(mx4[t], __uint_as_float(v[ch][j + 2 * t]), __uint_as_float(v[ch][j + 2 * t + 1]));
-        }
-      }
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      mx *= c;                                  // scale > 0
-      float alpha = 1.f;
-      if (mx - m > kLazy) {                     // also taken when m is still -inf
-        alpha = fast_exp2(m - mx);              // 0 when m was -inf
-        m = mx;
-      }
-      // Rescale this group's accumulator when some row of the warp moved its reference maximum.  The group's
-      // previous P V was issued before the scores that have just arrived and tcgen05.commit covers everything
-      // issued before it: that product has completed.
-      if (it > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-#pragma unroll 1
-        for (int ch = 0; ch < D / 16; ++ch) {     // rare: kept small, the 128 scores of the row stay in registers
-          uint32_t o[16];
-          tmem_ld16(tOg + ch * 16, o);
-          tmem_ld_wait16(o);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-          tmem_st16(tOg + ch * 16, o);
-        }
-      }
-      const float neg_m = (m == -INFINITY) ? 0.f : -m;
-      FPH(2)
-      float rs4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        uint32_t pk[16];
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(v[ch][j]), c, neg_m));       // exp2(-inf) = 0 on masked columns
-          const float p1 = fast_exp2(fmaf(__uint_as_float(v[ch][j + 1]), c, neg_m));
-          rs4[(j >> 1) & 3] += p0 + p1;
-          pk[j >> 1] = pack16<kF16>(p0, p1);
-        }
-        if (ch == 2) {                          // the first half of P (and the rescaled accumulator) is in TMEM by now
-          FPH(3)
-          tmem_st_wait();
-          tc_fence_before();
-          mbar_arrive(&bars[B_PFULL0 + wg]);
-          FPH(4)
-        }
-        tmem_st16(tS + ch * 16, pk);
-      }
-      const float rowsum = (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
-      l = l * alpha + rowsum;
-      FPH(5)
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars[B_PREST0 + wg]);
-      FPH(6)
-    }
-    if ((warp & 3) == 0) { FPH_END(wg, count) }
-
-    // ---- epilogue of this group: normalise and store its tile.  A barrier of its own that completes once
-    // tells that the group's last P V (and with it every MMA into its accumulator) has completed.
-    if (count > 0) {
-      if (ok) ok = mbar_wait(&bars[B_DONE0 + wg], 0, abort_flag, a.status, B_DONE0 + wg);
-      if (ok) {
+        FPH(0)
+        ok = mbar_wait(&bars[B_SFULL0 + wg], tiles & 1, abort_flag, a.status, B_SFULL0 + wg);
+        ok = __all_sync(0xffffffffu, ok);         // the warp leaves the loop together (warp-wide votes below)
+        FPH(1)
+        if (!ok) break;
         tc_fence_after();
-        const float inv = (l > 0.f) ? (1.f / l) : 0.f;     // a row that saw no unmasked key: O = 0
+
+        // All 128 scores of the row are read into registers with four back-to-back TMEM loads
+        // (one round trip), reduced to the row maximum, exponentiated in place and written back
+        // as P (bf16 pairs) over the first 64 score columns.
+        uint32_t v[4][32];
 #pragma unroll
-        for (int ch = 0; ch < D / 32; ++ch) {
-          uint32_t o[32];
-          tmem_ld32(tOg + ch * 32, o);
-          tmem_ld_wait(o);
-          if (row_valid) {
+        for (int ch = 0; ch < 4; ++ch) tmem_ld32(tS + ch * 32, v[ch]);
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // independent chains: no serial dependency
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint4 w4;
-              w4.x = pack16<kF16>(__uint_as_float(o[j + 0]) * inv, __uint_as_float(o[j + 1]) * inv);
-              w4.y = pack16<kF16>(__uint_as_float(o[j + 2]) * inv, __uint_as_float(o[j + 3]) * inv);
-              w4.z = pack16<kF16>(__uint_as_float(o[j + 4]) * inv, __uint_as_float(o[j + 5]) * inv);
-              w4.w = pack16<kF16>(__uint_as_float(o[j + 6]) * inv, __uint_as_float(o[j + 7]) * inv);
-              reinterpret_cast<uint4*>(o_row)[(ch * 32 + j) >> 3] = w4;
-            }
+        for (int ch = 0; ch < 4; ++ch) tmem_ld_wait(v[ch]);
+        if (partial) mask_scores(v, keep);        // in one block, off the path of whole tiles
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+              mx4[t] = fmax3(mx4[t], __uint_as_float(v[ch][j + 2 * t]), __uint_as_float(v[ch][j + 2 * t + 1]));
           }
         }
-        // A row that saw no unmasked key gets LSE2 = +inf, so that the backward pass computes
-        // exp2(s - LSE2) = 0 for it.
-        if (row_valid) *lse_row = (l > 0.f) ? (m + __log2f(l)) : INFINITY;
+        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        mx *= c;                                  // scale > 0
+        float alpha = 1.f;
+        if (mx - m > kLazy) {                     // also taken when m is still -inf
+          alpha = fast_exp2(m - mx);              // 0 when m was -inf
+          m = mx;
+        }
+        // Rescale this group's accumulator when some row of the warp moved its reference maximum.  The group's
+        // previous P V was issued before the scores that have just arrived and tcgen05.commit covers everything
+        // issued before it: that product has completed.
+        if (it > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+          for (int ch = 0; ch < D / 16; ++ch) {     // rare: kept small, the 128 scores of the row stay in registers
+            uint32_t o[16];
+            tmem_ld16(tOg + ch * 16, o);
+            tmem_ld_wait16(o);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+            tmem_st16(tOg + ch * 16, o);
+          }
+        }
+        const float neg_m = (m == -INFINITY) ? 0.f : -m;
+        FPH(2)
+        float rs4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float p0 = fast_exp2(fmaf(__uint_as_float(v[ch][j]), c, neg_m));       // exp2(-inf) = 0 on masked columns
+            const float p1 = fast_exp2(fmaf(__uint_as_float(v[ch][j + 1]), c, neg_m));
+            rs4[(j >> 1) & 3] += p0 + p1;
+            pk[j >> 1] = pack16<kF16>(p0, p1);
+          }
+          if (ch == 2) {                          // the first half of P (and the rescaled accumulator) is in TMEM by now
+            FPH(3)
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(&bars[B_PFULL0 + wg]);
+            FPH(4)
+          }
+          tmem_st16(tS + ch * 16, pk);
+        }
+        const float rowsum = (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
+        l = l * alpha + rowsum;
+        FPH(5)
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&bars[B_PREST0 + wg]);
+        FPH(6)
+      }
+
+      // ---- end of the piece for this group: normalise and store its tile.  The barrier tells that the group's last P V (and
+      // with it every MMA into its accumulator) has completed; the next piece's first P V waits for this group's next P.
+      {
+        if (ok) ok = mbar_wait(&bars[B_DONE0 + wg], uint32_t(pieces) & 1u, abort_flag, a.status, B_DONE0 + wg);
+        ok = __all_sync(0xffffffffu, ok);
+        ++pieces;
+        if (ok) {
+          tc_fence_after();
+          const float inv = (l > 0.f) ? (1.f / l) : 0.f;     // a row that saw no unmasked key: O = 0
+#pragma unroll
+          for (int ch = 0; ch < D / 32; ++ch) {
+            uint32_t o[32];
+            tmem_ld32(tOg + ch * 32, o);
+            tmem_ld_wait(o);
+            if (row_valid) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 8) {
+                uint4 w4;
+                w4.x = pack16<kF16>(__uint_as_float(o[j + 0]) * inv, __uint_as_float(o[j + 1]) * inv);
+                w4.y = pack16<kF16>(__uint_as_float(o[j + 2]) * inv, __uint_as_float(o[j + 3]) * inv);
+                w4.z = pack16<kF16>(__uint_as_float(o[j + 4]) * inv, __uint_as_float(o[j + 5]) * inv);
+                w4.w = pack16<kF16>(__uint_as_float(o[j + 6]) * inv, __uint_as_float(o[j + 7]) * inv);
+                reinterpret_cast<uint4*>(o_row)[(ch * 32 + j) >> 3] = w4;
+              }
+            }
+          }
+          // A row that saw no unmasked key gets LSE2 = +inf, so that the backward pass computes
+          // exp2(s - LSE2) = 0 for it.
+          if (row_valid) *lse_row = (l > 0.f) ? (m + __log2f(l)) : INFINITY;
+        }
       }
     }
+    if ((warp & 3) == 0) { FPH_END(wg, tiles) }
   }
 
   // ---------------------------------------------------------------------- teardown
@@ -554,8 +614,11 @@ namespace {
 template <int D, bool kF16>
 int launch_pairs(const FwdLaunch& L, cudaStream_t stream) {
   const FwdArgs& a = L.args;
-  // one CTA per pair of query tiles and head, or per query tile and pair of heads
-  dim3 grid(a.pair_heads ? a.list.n_outer_tiles * L.batch * (a.q_heads / 2) : ((a.list.n_outer_tiles + 1) / 2) * L.batch * a.q_heads, 1, 1);
+  // a piece of work per pair of query tiles and head, or per query tile and pair of heads
+  const long long work = a.pair_heads ? (long long)a.list.n_outer_tiles * L.batch * (a.q_heads / 2)
+                                      : (long long)((a.list.n_outer_tiles + 1) / 2) * L.batch * a.q_heads;
+  if (work > INT_MAX - 1024) return KVAX_B200_EUNSUPPORTED;
+  dim3 grid(int(work < kPersistentCtas ? work : kPersistentCtas), 1, 1);
   constexpr int smem = FwdSmem<D>::kTotal;
   auto kern = attn_fwd_kernel<D, kF16>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return KVAX_B200_ELAUNCH;

@@ -28,6 +28,7 @@
 // input dtype before P V, O = acc / l, LSE2 = m + log2(l); query tiles with no work get
 // O = 0 and LSE2 = 0 (:253-258).
 #include "attn_common.cuh"
+#include "attn_fwd_mask.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -69,7 +70,7 @@ struct FwdSmem {
 template <int D, bool kF16>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                const __grid_constant__ CUtensorMap tmap_v, const FwdArgs a) {
+                const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ FwdArgs a) {
   using L = FwdSmem<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -232,15 +233,6 @@ attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint32_t tS = tmem_base + wg * kTile + lane_base;
     const uint32_t tOg = tO + wg * kTile + lane_base;
     const float c = a.scale_log2e;
-    RowBounds rb = load_bounds(a.mask, b, min(r, a.tok.q_len - 1));
-    int q_seg = KVAX_B200_PADDING_SEGMENT_ID, q_pos = 0;
-    if (row_valid) {
-      q_seg = __ldg(a.tok.q_seg + (long long)b * a.tok.q_len + r);
-      q_pos = query_position(a.tok, b, r);
-    }
-    const int32_t* kv_seg = a.tok.kv_seg + (long long)b * a.tok.kv_len;
-    const int32_t* kv_pos = a.tok.kv_pos + (long long)b * a.tok.kv_len;
-
     // Online softmax state of this group.  `m` is the reference maximum the exponentials
     // use.  It only follows the true running maximum when that has grown by more than kLazy
     // (log2 units): P then stays below 2^kLazy and the accumulator in TMEM needs no rescaling
@@ -252,22 +244,9 @@ attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     for (int it = wg; it < count && ok; it += 2) {
       const uint32_t e = e_next;
       if (it + 2 < count) e_next = ldg_pinned(list + it + 2);
-      const int c0 = int(e & a.list.tile_mask) * kTile;
       const bool partial = (e & kPartialBit) != 0;
-
-      // element mask of partial tiles (computed before the scores arrive)
-      uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-      if (partial) {
-        if (e & kBitmapBit) {                   // worked out once by the list builder for every head: 16 bytes per row
-          const uint4 w = __ldg(entry_bitmap(a.list, e) + row);
-          keep[0] = w.x; keep[1] = w.y; keep[2] = w.z; keep[3] = w.w;
-        } else {
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch)
-            keep[ch] = keep_bits32<false>(rb, c0 + ch * 32, a.tok.kv_len, row_valid, q_seg, q_pos, kv_seg + c0 + ch * 32,
-                                          a.tok.sequential ? nullptr : kv_pos + c0 + ch * 32);
-        }
-      }
+      uint4 keep = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+      if (partial) keep = fwd_keep(a, e, b, r, row);           // fetched before the scores arrive
       ok = mbar_wait(&bars[B_SFULL0 + wg], (it >> 1) & 1, abort_flag, a.status, B_SFULL0 + wg);
       if (!ok) break;
       tc_fence_after();
@@ -280,12 +259,10 @@ attn_fwd_one_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       for (int ch = 0; ch < 4; ++ch) tmem_ld32(tS + ch * 32, v[ch]);
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // independent chains: no serial dependency
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        tmem_ld_wait(v[ch]);
-        if (partial) {
+      for (int ch = 0; ch < 4; ++ch) tmem_ld_wait(v[ch]);
+      if (partial) mask_scores(v, keep);          // in one block, off the path of whole tiles
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[ch][j] = ((keep[ch] >> j) & 1u) ? v[ch][j] : 0xff800000u;   // -inf
-        }
+      for (int ch = 0; ch < 4; ++ch) {
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
 #pragma unroll

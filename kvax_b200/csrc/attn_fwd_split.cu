@@ -23,6 +23,7 @@
 //
 // Semantics as attn_fwd_one.cu (kvax/ops/flash_attention_triton.py:137-370).
 #include "attn_common.cuh"
+#include "attn_fwd_mask.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -102,25 +103,6 @@ struct SegWalk {
     len = min(count, left);
   }
 };
-
-// Mask bits of query token r for the 128 keys from c0 of a partial list entry without an element mask (the pool of masks was
-// used up: rare).  Not inlined, so that what it needs lives in no register of the tile loop.
-__device__ __noinline__ uint4 split_keep_slow(const FwdArgs* a, int b, int r, bool row_valid, int c0) {
-  const RowBounds rb = load_bounds(a->mask, b, min(r, a->tok.q_len - 1));
-  int q_seg = KVAX_B200_PADDING_SEGMENT_ID, q_pos = 0;
-  if (row_valid) {
-    q_seg = __ldg(a->tok.q_seg + (long long)b * a->tok.q_len + r);
-    q_pos = query_position(a->tok, b, r);
-  }
-  const int32_t* kv_seg = a->tok.kv_seg + (long long)b * a->tok.kv_len;
-  const int32_t* kv_pos = a->tok.sequential ? nullptr : a->tok.kv_pos + (long long)b * a->tok.kv_len;
-  uint32_t w[4];
-#pragma unroll
-  for (int ch = 0; ch < 4; ++ch)
-    w[ch] = keep_bits32<false>(rb, c0 + ch * 32, a->tok.kv_len, row_valid, q_seg, q_pos, kv_seg + c0 + ch * 32,
-                               kv_pos ? kv_pos + c0 + ch * 32 : nullptr);
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
 
 template <int D, bool kF16>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -370,14 +352,9 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         const int t = t0 + i;
         const uint32_t e = e_next;
         if (i + 2 < sw.len) e_next = ldg_pinned(list + i + 2);
-        const int c0 = int(e & a.list.tile_mask) * kTile;
         const bool partial = (e & kPartialBit) != 0;
-        uint32_t keep[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-        if (partial && live) {
-          const uint4 w = (e & kBitmapBit) ? __ldg(entry_bitmap(a.list, e) + (tile_token & (kTile - 1)))
-                                           : split_keep_slow(&a, sw.b, r, row_valid, c0);
-          keep[0] = w.x; keep[1] = w.y; keep[2] = w.z; keep[3] = w.w;
-        }
+        uint4 keep = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        if (partial && live) keep = fwd_keep(a, e, sw.b, r, tile_token & (kTile - 1));
         ok = mbar_wait(&bars[B_SFULL0 + wg], (t >> 1) & 1, abort_flag, a.status, B_SFULL0 + wg);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -388,12 +365,10 @@ attn_fwd_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           for (int ch = 0; ch < 4; ++ch) tmem_ld32(tS + ch * 32, v[ch]);
           float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            tmem_ld_wait(v[ch]);
-            if (partial) {
+          for (int ch = 0; ch < 4; ++ch) tmem_ld_wait(v[ch]);
+          if (partial) mask_scores(v, keep);
 #pragma unroll
-              for (int jj = 0; jj < 32; ++jj) v[ch][jj] = ((keep[ch] >> jj) & 1u) ? v[ch][jj] : 0xff800000u;   // -inf
-            }
+          for (int ch = 0; ch < 4; ++ch) {
 #pragma unroll
             for (int jj = 0; jj < 32; jj += 8) {
 #pragma unroll

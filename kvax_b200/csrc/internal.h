@@ -54,6 +54,7 @@ struct FwdArgs {
   float* parts;             // (2 * kSplitCtas, 128, D) parts of items that several CTAs work on
   float2* part_ml;          // (2 * kSplitCtas, 128) their row maxima and sums
   int32_t* part_counters;   // (kSplitCtas) finished parts, zero on entry
+  int32_t* work_counter;    // pair kernel: pieces of work dealt out beyond the first of every CTA; zero between launches
   int32_t pair_heads;       // pair kernel: a CTA takes one query tile of two heads of a kv group instead of two tiles of one head
 };
 
