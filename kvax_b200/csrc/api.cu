@@ -282,14 +282,17 @@ extern "C" int kvax_b200_attn_fwd(const kvax_b200_attn_fwd_params* p, void* work
   a.scale_log2e = s.scale * 1.4426950408889634f;
   a.q_heads = s.q_heads; a.group = s.q_heads / s.kv_heads; a.batch = s.batch;
   L.batch = s.batch; L.head_dim = s.head_dim; L.dtype = s.dtype;
-  // Two work items per CTA that share their K / V tiles halve the K / V traffic and pay on long sequences; short ones
-  // have too few and too uneven CTAs that way (measured: 8k tokens 20 % slower, 16k dense 7-14 % faster).  With
-  // grouped-query attention the two items are one query tile of two heads of a kv group (identical tile lists), else
-  // two neighbouring query tiles of one head.
-  bool pairs = s.kv_len >= 16384;
-  // Head pairs have no one-sided entries and pay on shorter sequences too, as soon as the halved number of CTAs still
-  // fills the SMs twice over (measured, 32/8 heads: 8k tokens B=1 0.292 against 0.301 ms, B=4 0.97 / 1.06, 4k B=8 0.77 / 0.89).
-  if (s.q_heads / s.kv_heads % 2 == 0 && (long long)cdiv(s.q_len, kTile) * s.batch * (s.q_heads / 2) >= 2 * 148) pairs = true;
+  // Two work items that share their K / V tiles halve the K / V traffic: one query tile of two heads of a kv group (identical
+  // tile lists), or two neighbouring query tiles of one head.  One CTA per SM deals the pairs out, so they pay as soon as
+  // there are one and a half per SM (measured, us, one tile per CTA / pairs: 16/16 heads, 8 x 2112 tokens 157 / 126, head_dim 64
+  // 131 / 104, 1 x 8k 156 / 144; 6/2 heads 8 x 2000 59 / 53; 32/8 heads 1 x 8k 292 / 251, 1 x 2k, 256 pairs, 52 / 49; 2 x 1000
+  // tokens on 17k keys, 256 pairs, 542 / 525); below that SMs idle (6/2 heads 1 x 4000, 96 pairs, 35 / 49; 32/8 heads, 400
+  // tokens on 17k keys, 64 pairs, 150 / 281).  On long sequences, where a list may be as long as the sequence, the longest pair
+  // alone takes longer than an SM's share of the rest until there are two per SM (1 x 16k, 4/1 heads, 256 pairs, 193 / 207).
+  const long long n_tiles = cdiv(s.q_len, kTile);
+  const long long n_pairs = s.batch * (s.q_heads / s.kv_heads % 2 == 0 ? n_tiles * (s.q_heads / 2) : (n_tiles + 1) / 2 * s.q_heads);
+  const bool uneven = s.kv_len > 64 * kTile && 2ll * s.q_len > s.kv_len;
+  bool pairs = 2 * n_pairs >= (uneven ? 4 : 3) * kPersistentCtas;
   if (p->flags & KVAX_B200_FWD_ONE_TILE) pairs = false;
   if (p->flags & (KVAX_B200_FWD_TILE_PAIRS | KVAX_B200_FWD_HEAD_PAIRS)) pairs = true;
   a.empty_lse = (p->flags & KVAX_B200_FWD_EMPTY_LSE_INF) ? INFINITY : 0.f;
