@@ -7,6 +7,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libkvax_b200.so")
 
@@ -145,6 +147,23 @@ def load() -> C.CDLL:
     lib.kvax_b200_host_word_device_pointer.argtypes = [vp, C.POINTER(vp)]
     _lib = lib
     return lib
+
+
+def current_stream(device: torch.device) -> int:
+    """Handle of PyTorch's current stream on `device` (no Stream object is made for it)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+def launch(what: str, device: torch.device, *args) -> None:
+    """Calls the entry point `what` with `args` and the current stream of `device`, with that device current, and raises on
+    an error code."""
+    fn = getattr(load(), what)
+    if torch._C._cuda_getDevice() == device.index:
+        code = fn(*args, current_stream(device))
+    else:
+        with torch.cuda.device(device):
+            code = fn(*args, current_stream(device))
+    check(code, what)
 
 
 def check(code: int, what: str) -> None:

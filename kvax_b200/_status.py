@@ -14,11 +14,16 @@ import torch
 from kvax_b200 import _lib
 
 _words: dict[int, tuple[torch.Tensor, int]] = {}
+_views: dict[int, C.c_int32] = {}              # the same words as plain integers, for a look that makes no tensor
+
+
+def word_index(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
 
 
 def status_word(device: torch.device) -> tuple[torch.Tensor, int]:
     """(pinned host int32[1], address of that word as the device sees it)."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
+    idx = word_index(device)
     entry = _words.get(idx)
     if entry is None:
         word = torch.zeros(1, dtype=torch.int32).pin_memory()
@@ -28,6 +33,7 @@ def status_word(device: torch.device) -> tuple[torch.Tensor, int]:
         _lib.check(rc, "kvax_b200_host_word_device_pointer")
         entry = (word, int(dev_ptr.value))
         _words[idx] = entry
+        _views[idx] = C.c_int32.from_address(word.data_ptr())
     return entry
 
 
@@ -45,10 +51,13 @@ def check_last_status(device: torch.device | None = None, synchronize: bool = Fa
         device = torch.device("cuda", torch.cuda.current_device())
     if synchronize:
         torch.cuda.synchronize(device)
-    word, _ = status_word(device)
-    code = int(word[0])
+    view = _views.get(device.index)
+    if view is None:
+        word, _ = status_word(device)
+        view = _views[word_index(device)]
+    code = view.value
     if code != 0:
-        word[0] = 0
+        view.value = 0
         what = "the shared memory window was misaligned" if code == 90 else "a bounded wait gave up (100 + barrier id)"
         raise _lib.KvaxB200Error(f"attention kernel on {device} reported status {code}: {what}; "
                                  "outputs of that call are not valid")

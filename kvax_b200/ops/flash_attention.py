@@ -129,9 +129,7 @@ def _abs_max(*tensors) -> torch.Tensor:
     out = torch.empty(1, dtype=torch.float32, device=device)
     ptrs = (_lib.vp * len(ts))(*(t.data_ptr() for t in ts))
     sizes = (_lib.i64 * len(ts))(*(t.numel() for t in ts))
-    with torch.cuda.device(device):
-        rc = _lib.load().kvax_b200_abs_max(ptrs, sizes, len(ts), out.data_ptr(), torch.cuda.current_stream(device).cuda_stream)
-    _lib.check(rc, "kvax_b200_abs_max")
+    _lib.launch("kvax_b200_abs_max", device, ptrs, sizes, len(ts), out.data_ptr())
     return out
 
 
@@ -160,11 +158,9 @@ class _ToOperand(torch.autograd.Function):
         inv = ctx.box.inv
         if g.is_cuda and ctx.in_dtype == torch.float32 and g.dtype in (torch.float16, torch.bfloat16) and g.is_contiguous() and g.numel():
             out = torch.empty_like(g, dtype=torch.float32)
-            with torch.cuda.device(g.device):
-                rc = _lib.load().kvax_b200_widen_to_float(g.data_ptr(), g.numel(), _lib.DTYPE_F16 if g.dtype == torch.float16 else _lib.DTYPE_BF16,
-                                                          None if inv is None else inv.data_ptr(), out.data_ptr(),
-                                                          torch.cuda.current_stream(g.device).cuda_stream)
-            _lib.check(rc, "kvax_b200_widen_to_float")
+            dtype = _lib.DTYPE_F16 if g.dtype == torch.float16 else _lib.DTYPE_BF16
+            _lib.launch("kvax_b200_widen_to_float", g.device, g.data_ptr(), g.numel(), dtype, None if inv is None else inv.data_ptr(),
+                        out.data_ptr())
             return out, None, None
         g = g.to(ctx.in_dtype)
         if inv is not None:
@@ -191,10 +187,8 @@ class _FromOperand(torch.autograd.Function):
         amax = _abs_max(g)
         out = torch.empty_like(g, dtype=torch.float16)
         inv = torch.empty_like(amax)
-        with torch.cuda.device(g.device):
-            rc = _lib.load().kvax_b200_scale_to_operand(g.data_ptr(), g.numel(), amax.data_ptr(), _lib.DTYPE_F16, out.data_ptr(),
-                                                        inv.data_ptr(), torch.cuda.current_stream(g.device).cuda_stream)
-        _lib.check(rc, "kvax_b200_scale_to_operand")
+        _lib.launch("kvax_b200_scale_to_operand", g.device, g.data_ptr(), g.numel(), amax.data_ptr(), _lib.DTYPE_F16, out.data_ptr(),
+                    inv.data_ptr())
         ctx.box.inv = inv
         return out, None, None
 
@@ -251,11 +245,15 @@ def phase_times_ms() -> dict[str, float]:
     return out
 
 
-@contextlib.contextmanager
+_no_phase = contextlib.nullcontext()
+
+
 def _phase(name: str):
-    if _phase_log is None:
-        yield
-        return
+    return _no_phase if _phase_log is None else _timed_phase(name)
+
+
+@contextlib.contextmanager
+def _timed_phase(name: str):
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
     try:
@@ -290,7 +288,7 @@ _workspaces: dict[tuple, torch.Tensor] = {}
 
 
 def _workspace(kind: str, nbytes: int, device: torch.device) -> torch.Tensor:
-    key = (kind, device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (kind, device.index, _lib.current_stream(device))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
@@ -303,34 +301,32 @@ _KERNEL_HEAD_DIMS = (64, 128)                         # what the sm_100a kernels
 
 
 def _i32(x):
-    return x.to(torch.int32).contiguous()
+    return x if x.dtype == torch.int32 and x.is_contiguous() else x.to(torch.int32).contiguous()
 
 
 def _block_mask(mask: AttentionMask, q_block: int, kv_block: int) -> tuple[_lib.BlockMask, list]:
-    keep = [t.to(torch.int32).contiguous() for t in mask.flatten()]
-    bm = _lib.BlockMask()
-    bm.lower, bm.upper, bm.lower_full, bm.upper_full = (t.data_ptr() for t in keep)
-    bm.q_block, bm.kv_block = int(q_block), int(kv_block)
+    keep = [_i32(t) for t in mask.flatten()]
+    lower, upper, lower_full, upper_full = keep
+    bm = _lib.BlockMask(lower.data_ptr(), upper.data_ptr(), lower_full.data_ptr(), upper_full.data_ptr(), int(q_block), int(kv_block))
     return bm, keep
 
 
-def _fill_shape(s: _lib.AttnShape, q, k, v, o, q_pos, q_seg, kv_pos, kv_seg, scale, sequential, offsets):
+def _shape(q, k, v, o, q_pos, q_seg, kv_pos, kv_seg, scale, sequential, offsets) -> _lib.AttnShape:
     B, Sq, Hq, D = q.shape
-    s.batch, s.q_len, s.kv_len = B, Sq, k.shape[1]
-    s.q_heads, s.kv_heads, s.head_dim = Hq, k.shape[2], D
+    Skv, Hkv = k.shape[1], k.shape[2]
     if q.dtype not in (torch.bfloat16, torch.float16) or k.dtype != q.dtype or v.dtype != q.dtype:
         raise _lib.KvaxB200Error(f"the kernels take bf16 or fp16 operands of one type, got {q.dtype}, {k.dtype}, {v.dtype}")
-    s.dtype = _lib.DTYPE_F16 if q.dtype == torch.float16 else _lib.DTYPE_BF16
-    s.assume_sequential_positions = int(bool(sequential))
-    s.scale = float(scale)
-    for name, t in (("q_strides", q), ("k_strides", k), ("v_strides", v), ("o_strides", o)):
-        if t.stride(3) != 1:
-            raise AssertionError("head_dim must be contiguous")
-        arr = getattr(s, name)
-        arr[0], arr[1], arr[2] = t.stride(0), t.stride(1), t.stride(2)
-    s.q_positions, s.q_segment_ids = q_pos.data_ptr(), q_seg.data_ptr()
-    s.kv_positions, s.kv_segment_ids = kv_pos.data_ptr(), kv_seg.data_ptr()
-    s.q_global_offset_first, s.q_global_offset_second = offsets
+    strides = [t.stride() for t in (q, k, v, o)]
+    if any(st[3] != 1 for st in strides):
+        raise AssertionError("head_dim must be contiguous")
+    # the fields in the header's order: one construction instead of an attribute access each
+    return _lib.AttnShape(B, Sq, Skv, Hq, Hkv, D, _lib.DTYPE_F16 if q.dtype == torch.float16 else _lib.DTYPE_BF16,
+                          int(bool(sequential)), float(scale), 0, *(st[:3] for st in strides), q_pos.data_ptr(), q_seg.data_ptr(),
+                          kv_pos.data_ptr(), kv_seg.data_ptr(), *offsets)
+
+
+_FWD_FLAGS = {"auto": 0, "one_tile": _lib.FWD_ONE_TILE, "tile_pairs": _lib.FWD_TILE_PAIRS, "head_pairs": _lib.FWD_HEAD_PAIRS,
+              "split": _lib.FWD_SPLIT}
 
 
 def attention_forward(q, k, v, q_pos, q_seg, kv_pos, kv_seg, mask_fwd: AttentionMask, fwd_blocks, scale,
@@ -345,22 +341,17 @@ def attention_forward(q, k, v, q_pos, q_seg, kv_pos, kv_seg, mask_fwd: Attention
     out = torch.empty_like(q) if out is None else out
     lse = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device) if lse is None else lse
     status, status_ptr = status_word(q.device)
-    p = _lib.AttnFwdParams()
-    p.stages = int(stages)
-    p.flags = {"auto": 0, "one_tile": _lib.FWD_ONE_TILE, "tile_pairs": _lib.FWD_TILE_PAIRS,
-               "head_pairs": _lib.FWD_HEAD_PAIRS, "split": _lib.FWD_SPLIT}[kernel or _fwd_kernel] | (_lib.FWD_EMPTY_LSE_INF if empty_lse_inf else 0)
-    _fill_shape(p.shape, q, k, v, out, q_pos, q_seg, kv_pos, kv_seg, scale, assume_sequential_positions, offsets)
-    p.q, p.k, p.v = q.data_ptr(), k.data_ptr(), v.data_ptr()
-    p.mask, keep = _block_mask(mask_fwd, *fwd_blocks)
-    p.out, p.lse, p.status = out.data_ptr(), lse.data_ptr(), status_ptr
+    mask, keep = _block_mask(mask_fwd, *fwd_blocks)
+    p = _lib.AttnFwdParams(
+        _shape(q, k, v, out, q_pos, q_seg, kv_pos, kv_seg, scale, assume_sequential_positions, offsets),
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), mask, out.data_ptr(), lse.data_ptr(), status_ptr, int(stages),
+        _FWD_FLAGS[kernel or _fwd_kernel] | (_lib.FWD_EMPTY_LSE_INF if empty_lse_inf else 0))
     ws_bytes = lib.kvax_b200_attn_fwd_workspace_bytes(p)
     if ws_bytes == 0:
         raise _lib.KvaxB200Error("kvax_b200_attn_fwd_workspace_bytes rejected the arguments "
                                  f"(head_dim={D}, dtype={q.dtype})")
     ws = _workspace("fwd", ws_bytes, q.device) if workspace is None else workspace
-    with torch.cuda.device(q.device):
-        rc = lib.kvax_b200_attn_fwd(p, ws.data_ptr(), ws.numel(), torch.cuda.current_stream(q.device).cuda_stream)
-    _lib.check(rc, "kvax_b200_attn_fwd")
+    _lib.launch("kvax_b200_attn_fwd", q.device, p, ws.data_ptr(), ws.numel())
     if workspace is not None or stages:
         return out, lse, status, ws
     return out, lse, status
@@ -382,28 +373,24 @@ def attention_backward(q, k, v, out, dout, lse, q_pos, q_seg, kv_pos, kv_seg, ma
     else:
         dq, dk, dv = grads
     status, status_ptr = status_word(q.device)
-    p = _lib.AttnBwdParams()
-    p.stages = int(stages)
-    p.flags = (_lib.BWD_TWO_KERNEL if (mode or _bwd_mode) == "two_kernel" else 0) | (_lib.BWD_DKDV_16BIT if dkdv_in_operand_dtype else 0)
     if out.stride() != dout.stride():
         dout = dout.contiguous()
         out = out.contiguous()
-    _fill_shape(p.shape, q, k, v, out, q_pos, q_seg, kv_pos, kv_seg, scale, assume_sequential_positions, offsets)
-    if dq.stride(3) != 1:
+    shape = _shape(q, k, v, out, q_pos, q_seg, kv_pos, kv_seg, scale, assume_sequential_positions, offsets)
+    dq_strides = dq.stride()
+    if dq_strides[3] != 1:
         raise AssertionError("head_dim of dq must be contiguous")
-    p.dq_strides[0], p.dq_strides[1], p.dq_strides[2] = dq.stride(0), dq.stride(1), dq.stride(2)
-    p.q, p.k, p.v, p.out, p.dout, p.lse = (t.data_ptr() for t in (q, k, v, out, dout, lse))
     bq, bk = bwd_blocks
-    p.mask_dq, keep1 = _block_mask(mask_dq, bk, bq)        # dq mask: block sizes swapped
-    p.mask_dkdv, keep2 = _block_mask(mask_dkdv, bq, bk)
-    p.dq, p.dk, p.dv, p.status = dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), status_ptr
+    m_dq, keep1 = _block_mask(mask_dq, bk, bq)             # dq mask: block sizes swapped
+    m_dkdv, keep2 = _block_mask(mask_dkdv, bq, bk)
+    flags = (_lib.BWD_TWO_KERNEL if (mode or _bwd_mode) == "two_kernel" else 0) | (_lib.BWD_DKDV_16BIT if dkdv_in_operand_dtype else 0)
+    p = _lib.AttnBwdParams(shape, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),
+                           m_dq, m_dkdv, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), status_ptr, int(stages), flags, dq_strides[:3])
     ws_bytes = lib.kvax_b200_attn_bwd_workspace_bytes(p)
     if ws_bytes == 0:
         raise _lib.KvaxB200Error("kvax_b200_attn_bwd_workspace_bytes rejected the arguments")
     ws = _workspace("bwd", ws_bytes, q.device) if workspace is None else workspace
-    with torch.cuda.device(q.device):
-        rc = lib.kvax_b200_attn_bwd(p, ws.data_ptr(), ws.numel(), torch.cuda.current_stream(q.device).cuda_stream)
-    _lib.check(rc, "kvax_b200_attn_bwd")
+    _lib.launch("kvax_b200_attn_bwd", q.device, p, ws.data_ptr(), ws.numel())
     if workspace is not None or stages:
         return dq, dk, dv, status, ws
     return dq, dk, dv, status

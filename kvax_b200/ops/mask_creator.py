@@ -60,23 +60,19 @@ class MaskPlan:
         self._keep = (qp, qs, kp, ks)
         self._lib = _lib.load()
         self.device = qp.device
-        p = self.params = _lib.MaskParams()
-        p.q_positions, p.q_segment_ids = qp.data_ptr(), qs.data_ptr()
-        p.kv_positions, p.kv_segment_ids = kp.data_ptr(), ks.data_ptr()
-        p.batch, p.q_len, p.kv_len = B, Sq, Skv
-        p.skip_pad_tokens = int(bool(skip_pad_tokens))
-        p.n_masks = len(block_specs)
-        for i, (bq, bk, kv_outer) in enumerate(block_specs):
-            d = p.masks[i]
-            d.q_block, d.kv_block, d.kv_outer = int(bq), int(bk), int(bool(kv_outer))
-        key = (B, Sq, Skv, tuple((int(bq), int(bk), bool(kv)) for bq, bk, kv in block_specs))
+        specs = [(int(bq), int(bk), bool(kv_outer)) for bq, bk, kv_outer in block_specs]
+        p = self.params = _lib.MaskParams(qp.data_ptr(), qs.data_ptr(), kp.data_ptr(), ks.data_ptr(), B, Sq, Skv,
+                                          int(bool(skip_pad_tokens)), len(specs))
+        key = (B, Sq, Skv, tuple(specs))
         layout = _layouts.get(key)
         if layout is None:
+            for i, (bq, bk, kv_outer) in enumerate(specs):
+                p.masks[i] = _lib.MaskDesc(bq, bk, kv_outer)
             ws_bytes = self._lib.kvax_b200_mask_workspace_bytes(p)
             if ws_bytes == 0:
                 raise _lib.KvaxB200Error("kvax_b200_mask_workspace_bytes rejected the arguments")
             # one int32 allocation holds the workspace and every output array (each output starts on a 256-byte boundary)
-            sizes = [(Skv + bk - 1) // bk if kv_outer else (Sq + bq - 1) // bq for (bq, bk, kv_outer) in block_specs]
+            sizes = [(Skv + bk - 1) // bk if kv_outer else (Sq + bq - 1) // bq for (bq, bk, kv_outer) in specs]
             offs, off = [], ((ws_bytes + 255) // 256) * 64            # in int32 elements
             for n in sizes:
                 offs.append(off)
@@ -86,20 +82,15 @@ class MaskPlan:
         self._blob = torch.empty(total, dtype=torch.int32, device=qp.device)
         base = self._blob.data_ptr()
         masks = []
-        for i, (n, off) in enumerate(zip(sizes, offs)):
-            arrs = self._blob[off:off + 4 * B * n].view(4, B, 1, n).unbind(0)
-            d = p.masks[i]
-            step = 4 * B * n
-            d.lower, d.upper, d.lower_full, d.upper_full = (base + 4 * off, base + 4 * off + step,
-                                                            base + 4 * off + 2 * step, base + 4 * off + 3 * step)
-            masks.append(AttentionMask(arrs[0], arrs[1], arrs[2], arrs[3]))
+        for i, (spec, n, off) in enumerate(zip(specs, sizes, offs)):
+            step = B * n
+            masks.append(AttentionMask(*self._blob.as_strided((4, B, 1, n), (step, n, n, 1), off).unbind(0)))
+            at, step = base + 4 * off, 4 * step
+            p.masks[i] = _lib.MaskDesc(*spec, 0, at, at + step, at + 2 * step, at + 3 * step)
         self.masks = tuple(masks)
 
     def launch(self) -> tuple[AttentionMask, ...]:
-        with torch.cuda.device(self.device):
-            rc = self._lib.kvax_b200_mask_build(self.params, self._blob.data_ptr(), self.ws_bytes,
-                                                torch.cuda.current_stream(self.device).cuda_stream)
-        _lib.check(rc, "kvax_b200_mask_build")
+        _lib.launch("kvax_b200_mask_build", self.device, self.params, self._blob.data_ptr(), self.ws_bytes)
         return self.masks
 
 

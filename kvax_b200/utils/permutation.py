@@ -42,11 +42,7 @@ def _permute_one(x: torch.Tensor, cp: int, reverse: bool) -> torch.Tensor:
     row_bytes = x.element_size()
     for d in x.shape[2:]:
         row_bytes *= d
-    stream = torch.cuda.current_stream(x.device).cuda_stream
-    with torch.cuda.device(x.device):
-        rc = _lib.load().kvax_b200_permute_tokens(x.data_ptr(), out.data_ptr(), x.shape[0], x.shape[1], row_bytes,
-                                                  cp, int(reverse), stream)
-    _lib.check(rc, "kvax_b200_permute_tokens")
+    _lib.launch("kvax_b200_permute_tokens", x.device, x.data_ptr(), out.data_ptr(), x.shape[0], x.shape[1], row_bytes, cp, int(reverse))
     return out
 
 
