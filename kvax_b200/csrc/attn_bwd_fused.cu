@@ -550,19 +550,24 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         uint32_t v[2][32];
         tmem_ld32(my_t1, v[0]);
         tmem_ld32(my_t1 + 32, v[1]);
+        tmem_ld_wait(v[0]);
+        tmem_ld_wait(v[1]);
+        if (partial) {                              // in one block, off the path of whole tiles: exp2(-inf) = 0
+#pragma unroll
+          for (int ch = 0; ch < 2; ++ch) {
+#pragma unroll
+            for (int jj = 0; jj < 32; ++jj) v[ch][jj] = ((keep[ch] >> jj) & 1u) ? v[ch][jj] : 0xff800000u;
+          }
+        }
 #pragma unroll
         for (int ch = 0; ch < 2; ++ch) {
-          tmem_ld_wait(v[ch]);
 #pragma unroll
           for (int jj = 0; jj < 32; jj += 4) {
             const float4 ls = cs_lse[(ch * 32 + jj) >> 2];
             const float l4[4] = {ls.x, ls.y, ls.z, ls.w};
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              float pv = fast_exp2(fmaf(__uint_as_float(v[ch][jj + t]), c, -l4[t]));
-              if (partial) pv = ((keep[ch] >> (jj + t)) & 1u) ? pv : 0.f;
-              v[ch][jj + t] = __float_as_uint(pv);
-            }
+            for (int t = 0; t < 4; ++t)
+              v[ch][jj + t] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(v[ch][jj + t]), c, -l4[t])));
           }
           uint32_t pk[16];
 #pragma unroll
