@@ -316,17 +316,22 @@ bool use_fused(const kvax_b200_attn_bwd_params& p) {
   return !(p.flags & KVAX_B200_BWD_TWO_KERNEL) && attn_bwd_fused_supports(p.shape.head_dim);
 }
 
-// Fused backward: CTAs per (kv tile, kv head).  One CTA walks every query head of the kv head; when that gives few CTAs
-// (short sequences, few kv heads: one long CTA then holds up a whole launch) the query heads are divided over 2, 4, ...
-// CTAs whose dK / dV parts are summed in fp32 accumulators.
+// Fused backward: pieces of work per (kv tile, kv head).  One piece walks every query head of the kv head; when that makes few
+// pieces (short sequences, few kv heads) the query heads are divided over 2, 4, ... pieces whose dK / dV parts are summed in fp32
+// accumulators.  That costs the zero fill of the accumulators, the adds at the end of a piece and a pass to the output type.
 int fused_head_split(const kvax_b200_attn_shape& s) {
   const int group = s.q_heads / s.kv_heads;
-  const long long ctas = (long long)cdiv(s.kv_len, kTile) * s.batch * s.kv_heads;
+  const long long pieces = (long long)cdiv(s.kv_len, kTile) * s.batch * s.kv_heads;
   int split = 1;
-  // Measured: below 16 CTAs per SM the split pays whatever the group; up to 32 per SM it pays for CTAs that walk eight
-  // or more heads (128k tokens, 32/4 heads: 86.6 -> 82.9 ms) and costs 3 % for four (32k, 32/8 heads: the zero fill
-  // and the final pass over dK / dV outweigh the shorter tail).
-  while (group % (2 * split) == 0 && (ctas * split < 16 * 148 || (ctas * split < 32 * 148 && group / split >= 8))) split *= 2;
+  // Measured (us, all backward kernels, split 1 / 2 / 4, 32/8 heads): 4 x 4k tokens, 6.9 pieces per SM, 870 / 917 / 969; one row of 8k,
+  // 3.5, 653 / 659 / 671; 8 x 1024 at head_dim 64, 3.5, 167 / 190 / 210; 1 x 4k, 1.7, 317 / 319 / 316; 1 x 2k, 0.9, 159 / 146 / 135;
+  // 1 x 512, 0.2, 48 / 40 / 33: three pieces per SM are enough.  From 16k tokens on, a piece of eight or more heads is so long that
+  // the last ones hold up the launch until there are more than 32 per SM (16k, 32/4 heads 3380 / 3294; 64k, 8/1 heads 14915 / 13901;
+  // 128k, 32/4 heads 118.4 / 115.9 ms).
+  auto few = [&] {
+    return pieces * split < 3 * kPersistentCtas || (group / split >= 8 && s.kv_len >= 16384 && pieces * split < 32 * kPersistentCtas);
+  };
+  while (group % (2 * split) == 0 && few()) split *= 2;
   return split;
 }
 
