@@ -670,11 +670,11 @@ def main():
         return
 
     value = flops_step / (ms_step * 1e-3) / 1e12
-    # kernels of this library per step: mask builder (1), forward (tile summaries, lists, order, attention),
-    # backward (tile summaries, lists, order, delta + zero fill, fused kernel, dQ cast); with context parallelism the
+    # kernels of this library per step: mask builder (1), forward (tile summaries, lists, attention),
+    # backward (tile summaries, lists, delta + zero fill, fused kernel, dQ cast); with context parallelism the
     # head exchange adds the rebuilt masks (1), two token un-permutations and eight exchange kernels (q, k, v, o, do,
     # dq, dk, dv), the all-gather schedule four token (un-)permutations
-    kernels_per_step = 1 + 4 + 6 + (0 if cp == 1 else (11 if hx else 4))
+    kernels_per_step = 1 + 3 + 5 + (0 if cp == 1 else (11 if hx else 4))
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": cp, "steps": K, "warmup": W,
         "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
@@ -690,9 +690,11 @@ def main():
     if cp == 1:
         line["config"]["tile_pairs_in_reference_bounds"] = reference_visited
         # the library's default choice of forward kernel for this shape (see kvax_b200_attn_fwd_params.flags)
-        head_pairs = (Hq // Hkv) % 2 == 0 and (S // TILE) * B * (Hq // 2) >= 2 * 148
-        line["config"]["forward_kernel"] = ("two heads of a kv group per CTA" if head_pairs or (S >= 16384 and (Hq // Hkv) % 2 == 0) else
-                                            ("two query tiles per CTA" if S >= 16384 else "one query tile per CTA"))
+        pair_heads, n_tiles_q = (Hq // Hkv) % 2 == 0, -(-S // TILE)
+        n_pairs = B * (n_tiles_q * (Hq // 2) if pair_heads else (n_tiles_q + 1) // 2 * Hq)
+        pairs = 2 * n_pairs >= (4 if S > 64 * TILE else 3) * 148
+        line["config"]["forward_kernel"] = (("pairs of heads of a kv group" if pair_heads else "pairs of query tiles") if pairs else
+                                            "one query tile per CTA")
     if roofline:
         line["roofline"] = roofline
     if cp == 1 and mask_info:
